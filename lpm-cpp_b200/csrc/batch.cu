@@ -2116,10 +2116,11 @@ enum class Ph
     Newton,      // force state after a Newton update in flight
     NeedCG,      // a CG (FP64, or the FP32 inner solve of a refinement) to start or resume
     DamageCheck, // J2 state + static damage in flight
+    FlagWait,    // tangent mode: the flags of the K just assembled in flight (cluster members)
     Done,
     Failed
 };
-constexpr int kPhases = 7;
+constexpr int kPhases = 8;
 
 struct Member
 {
@@ -2154,7 +2155,13 @@ struct Member
     int64_t cost = 0;
     // solo: the member's linear solves run alone through the single-problem CG (solo_solves)
     bool solo = false;
-    int64_t lane_cost() const { return solo ? 0 : cost; }
+    // cluster: the member's problem fits one thread-block cluster in the bond form, so each of its
+    // linear solves is a launch of its own on its own stream, with the Newton update and the next
+    // force state enqueued behind it; its rounds wait for no other member.  A K without a bond form
+    // (Scalars::bond_flag) goes through the member's lane instead.
+    bool cluster = false;
+    bool solving = false; // such a solve is in flight
+    int64_t lane_cost() const { return solo || cluster ? 0 : cost; }
 };
 
 // A lane: a share of the SMs with its own batched CG launches (FP64 members, then the FP32 inner
@@ -2191,6 +2198,7 @@ struct lpmgpu_batch
     lpmgpu_batch_stats stats{};
     std::chrono::steady_clock::time_point t_create;
     int64_t round_max_it = 0; // most CG iterations one member ran in this round's launches
+    double cluster_seconds = 0; // device time of the cluster members' solves
 
     Problem &P(Member &m) { return m.h->p; }
 
@@ -2262,7 +2270,7 @@ struct lpmgpu_batch
 
     double kernel_seconds() const
     {
-        double t = 0;
+        double t = cluster_seconds;
         for (auto &L : lanes)
             t += L->c64.kernel_seconds + L->c32.kernel_seconds;
         return t;
@@ -2424,10 +2432,72 @@ struct lpmgpu_batch
         if (p.desc.tangent)
         {
             // tangent mode: K (and its FP32 copy) from the current state before every solve
-            const cudaError_t e0 = enqueue_assemble(p, true);
+            cudaError_t e0 = enqueue_assemble(p, true);
+            if (e0 == cudaSuccess && m.cluster)
+            {
+                e0 = cudaMemcpyAsync(p.scal_host, p.scal, sizeof(Scalars), cudaMemcpyDeviceToHost, p.stream);
+                m.ph = Ph::FlagWait;
+                m.pending = true;
+            }
             if (e0 != cudaSuccess)
                 return fail_member(m, cuda_status(e0, "batch tangent assembly"));
+            if (m.pending)
+                return LPMGPU_OK;
         }
+        return start_solve(m);
+    }
+
+    // A cluster member's solve, its Newton update and the next force state, in one go.
+    int32_t start_cluster_solve(Member &m)
+    {
+        Problem &p = P(m);
+        const int64_t maxit = p.desc.cg_maxit > 0 ? p.desc.cg_maxit : (int64_t)p.n * p.dim;
+        cudaError_t e = cudaEventRecord(p.cg_ev[0], p.stream);
+        if (e == cudaSuccess)
+            e = enqueue_bond_cluster(p, p.res, p.x, p.desc.cg_rtol, p.desc.cg_atol, -1.0, maxit);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(p.cg_ev[1], p.stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p.cg_info_host, p.cg_info, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, p.stream);
+        if (e != cudaSuccess)
+            return fail_member(m, cuda_status(e, "batched cluster solve"));
+        stats.cg_launches++;
+        m.solving = true;
+        return finish_linear(m);
+    }
+
+    // its result, once the member's stream has run dry; false when the solve timed out
+    bool take_cluster_solve(Member &m)
+    {
+        Problem &p = P(m);
+        m.solving = false;
+        float ms = 0;
+        if (cudaEventElapsedTime(&ms, p.cg_ev[0], p.cg_ev[1]) == cudaSuccess)
+        {
+            p.ctr.cg_kernel_seconds += ms * 1e-3;
+            cluster_seconds += ms * 1e-3;
+        }
+        const int64_t it = p.cg_info_host[0];
+        m.cur.cg_iters += it;
+        m.cur.cg_maxit_hits += (p.cg_info_host[1] & 1) ? 1 : 0;
+        m.cur.refinements += p.desc.precision == LPMGPU_MIXED ? 1 : 0; // one outer step, solved in FP64
+        m.dof_iters += it * (int64_t)p.n * p.dim;
+        p.ctr.cg_iters += it;
+        round_max_it = std::max(round_max_it, it);
+        if (p.cg_info_host[1] & 2)
+        {
+            set_last_error("a device-side wait timed out in the batched cluster solve");
+            fail_member(m, LPMGPU_ERR_TIMEOUT);
+            return false;
+        }
+        return true;
+    }
+
+    int32_t start_solve(Member &m)
+    {
+        Problem &p = P(m);
+        if (m.cluster && bond_cluster_fits(p) && (p.scal_host->bond_flag & bond_flags_bad(p)) == 0)
+            return start_cluster_solve(m);
         if (p.desc.precision != LPMGPU_MIXED || m.solo)
         {
             m.ph = Ph::NeedCG; // a solo member's solve sets up its own refinement
@@ -2464,10 +2534,14 @@ struct lpmgpu_batch
     {
         Problem &p = P(m);
         m.pending = false;
+        if (m.solving && !take_cluster_solve(m))
+            return LPMGPU_OK;
         if (p.scal_host->err)
             return fail_member(m, LPMGPU_ERR_TOPOLOGY);
         switch (m.ph)
         {
+        case Ph::FlagWait:
+            return start_solve(m);
         case Ph::NewtonFirst:
         {
             m.nres = std::sqrt(p.scal_host->res_sq);
@@ -2695,7 +2769,10 @@ struct lpmgpu_batch
     bool lane_ready(Lane &L)
     {
         const cudaEvent_t ev = !L.g32.empty() ? L.c32.ev_done : L.c64.ev_done;
-        return cudaEventQuery(ev) == cudaSuccess;
+        const bool ready = cudaEventQuery(ev) == cudaSuccess;
+        if (!ready)
+            (void)cudaGetLastError(); // "not ready" is no error of a later launch check
+        return ready;
     }
 
     int32_t complete_lane(Lane &L)
@@ -2714,14 +2791,14 @@ struct lpmgpu_batch
         for (int pass = 0; pass < 1000; ++pass)
         {
             for (auto &up : members)
-                if (up && up->lane == l && up->ph == Ph::Start)
+                if (up && up->lane == l && !up->cluster && up->ph == Ph::Start)
                 {
                     cudaSetDevice(P(*up).device);
                     begin_substep(*up);
                 }
             std::vector<Member *> pend;
             for (auto &up : members)
-                if (up && up->lane == l && up->pending)
+                if (up && up->lane == l && !up->cluster && up->pending)
                     pend.push_back(up.get());
             if (pend.empty())
                 break;
@@ -2730,6 +2807,41 @@ struct lpmgpu_batch
                 return cuda_status(e, "batch round");
             for (Member *m : pend)
                 resolve(*m);
+        }
+        return LPMGPU_OK;
+    }
+
+    // The cluster members: starts the next sub-step of each that waits for one and takes the results
+    // of each whose stream has run dry (which enqueues its next piece of work).  *ran: some did;
+    // *waiting: some have work in flight.
+    int32_t poll_cluster(bool *ran, bool *waiting)
+    {
+        *waiting = false;
+        for (auto &up : members)
+        {
+            if (!up || !up->cluster)
+                continue;
+            Member &m = *up;
+            if (m.pending)
+            {
+                const cudaError_t e = cudaStreamQuery(P(m).stream);
+                if (e == cudaErrorNotReady)
+                {
+                    (void)cudaGetLastError(); // not an error, and not a later launch check's
+                    *waiting = true;
+                    continue;
+                }
+                if (e != cudaSuccess)
+                    return cuda_status(e, "batch round");
+                resolve(m);
+                *ran = true;
+            }
+            while (m.ph == Ph::Start)
+            {
+                begin_substep(m);
+                *ran = true;
+            }
+            *waiting = *waiting || m.pending;
         }
         return LPMGPU_OK;
     }
@@ -2765,6 +2877,12 @@ struct lpmgpu_batch
             progressed = progressed || ran;
             solo_ms = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_solo).count() * 1e3;
         }
+        bool waiting = false;
+        {
+            const int32_t r = poll_cluster(&progressed, &waiting);
+            if (r != LPMGPU_OK)
+                return r;
+        }
         int launched = 0;
         for (int l = 0; l < (int)lanes.size(); ++l)
         {
@@ -2777,6 +2895,16 @@ struct lpmgpu_batch
                 return r;
             if (lanes[l]->inflight)
                 launched++;
+        }
+        while (!progressed && launched == 0 && waiting)
+        {
+            // wait for the next member or lane to finish its work
+            const int32_t r = poll_cluster(&progressed, &waiting);
+            if (r != LPMGPU_OK)
+                return r;
+            for (auto &L : lanes)
+                if (L->inflight && lane_ready(*L))
+                    progressed = true; // the next round takes its results
         }
         if (!progressed && launched == 0)
         {
@@ -2824,11 +2952,11 @@ struct lpmgpu_batch
                 infl += L->inflight ? 1 : 0;
             std::fprintf(stderr,
                          "lpmgpu batch round %lld: lanes in flight %d/%zu launches=%lld max_it=%lld kernel_ms=%.3f "
-                         "round_ms=%.3f solo_ms=%.3f phases(start,nf,n,cg,dmg,done,fail)=%d,%d,%d,%d,%d,%d,%d\n",
+                         "round_ms=%.3f solo_ms=%.3f phases(start,nf,n,cg,dmg,flag,done,fail)=%d,%d,%d,%d,%d,%d,%d,%d\n",
                          (long long)stats.rounds, infl, lanes.size(), (long long)(stats.cg_launches - l0),
                          (long long)round_max_it, (kernel_seconds() - k0) * 1e3,
                          std::chrono::duration<double>(std::chrono::steady_clock::now() - t_round).count() * 1e3,
-                         solo_ms, nph[0], nph[1], nph[2], nph[3], nph[4], nph[5], nph[6]);
+                         solo_ms, nph[0], nph[1], nph[2], nph[3], nph[4], nph[5], nph[6], nph[7]);
         }
         return LPMGPU_OK;
     }
@@ -2937,6 +3065,9 @@ static int32_t push_member(lpmgpu_batch *b, std::unique_ptr<Member> m, int32_t *
     const Problem &p = m->h->p;
     m->cost = p.nsb * (p.dim * p.dim + 1);
     m->solo = b->solo_bytes > 0 && cg_stream_bytes(p) >= b->solo_bytes;
+    // LPMGPU_BATCH_SR names the batched kernel of the mixed members: they then stay in their lanes
+    m->cluster = !m->solo && p.bo_ok && p.bo_nc > 0 && p.asm_fast && !p.asm_exact &&
+                 !(p.desc.precision == LPMGPU_MIXED && std::getenv("LPMGPU_BATCH_SR"));
     int best = 0;
     for (int l = 1; l < (int)b->lanes.size(); ++l)
         if (b->lanes[l]->cost < b->lanes[best]->cost)

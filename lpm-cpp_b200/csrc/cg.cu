@@ -31,6 +31,7 @@
 #include <vector>
 #include <string>
 
+#include "bond_op.cuh"
 #include "cg_device.cuh"
 
 namespace lpm
@@ -365,6 +366,44 @@ static cudaError_t cg_grid_rule(const Problem &p, int *grid_out)
     return cudaSuccess;
 }
 
+// Waits for the CG launch between the handle's two events and reads its status words.
+static cudaError_t finish_cg(Problem &p, const char *what, CGResult &out, double *rr_final, bool *declined)
+{
+    cudaError_t e;
+    if ((e = cudaEventRecord(p.cg_ev[1], p.stream)) != cudaSuccess)
+        return e;
+    if ((e = cudaMemcpyAsync(p.cg_info_host, p.cg_info, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, p.stream)) !=
+        cudaSuccess)
+        return e;
+    if ((e = cudaStreamSynchronize(p.stream)) != cudaSuccess)
+        return e;
+    if (declined && (p.cg_info_host[1] & kBondDeclined))
+    {
+        *declined = true;
+        return cudaSuccess;
+    }
+    out.iters += p.cg_info_host[0];
+    p.ctr.cg_iters += p.cg_info_host[0];
+    {
+        float ms = 0;
+        if (cudaEventElapsedTime(&ms, p.cg_ev[0], p.cg_ev[1]) == cudaSuccess)
+            p.ctr.cg_kernel_seconds += ms * 1e-3;
+        static const bool log = std::getenv("LPMGPU_LOG") != nullptr;
+        if (log)
+            std::fprintf(stderr, "lpmgpu cg launch %lld: %s/%dd n=%d iters=%lld ms=%.3f\n", (long long)p.ctr.cg_launches,
+                         what, p.dim, p.n, (long long)p.cg_info_host[0], ms);
+    }
+    if (p.cg_info_host[1] & 1)
+        out.maxit_hits++;
+    if (p.cg_info_host[1] & 2)
+        out.timeout = true;
+    if (p.cg_info_host[1] & 4)
+        out.breakdown = true;
+    if (rr_final)
+        *rr_final = reinterpret_cast<double *>(p.cg_info_host)[3];
+    return cudaSuccess;
+}
+
 template <typename TK, typename TV, int D>
 static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV *pa, TV *pb, TV *q, double rtol,
                           double atol, double abs_stop, int64_t maxit, CGResult &out, double *rr_final)
@@ -402,36 +441,37 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D>, dim3(grid), dim3(kCGThreads), args, 0, p.stream);
     if (e != cudaSuccess)
         return e;
-    if ((e = cudaEventRecord(p.cg_ev[1], p.stream)) != cudaSuccess)
-        return e;
     p.ctr.kernel_launches++;
     p.ctr.cg_launches++;
-    if ((e = cudaMemcpyAsync(p.cg_info_host, p.cg_info, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, p.stream)) !=
-        cudaSuccess)
+    return finish_cg(p, sizeof(TK) == 8 ? "assembled fp64" : "assembled fp32", out, rr_final, nullptr);
+}
+
+// K x = b on the bond form of the K assembled last (bond_op.cu), in one cluster when the problem fits
+// one, else on the whole grid.  *declined: this K has no bond form, nothing was solved.
+template <typename TV>
+static cudaError_t run_bond(Problem &p, const TV *b, TV *x, TV *r, TV *pa, TV *pb, double rtol, double atol,
+                            double abs_stop, int64_t maxit, CGResult &out, double *rr_final, bool *declined)
+{
+    cudaError_t e;
+    *declined = false;
+    if ((e = cudaEventRecord(p.cg_ev[0], p.stream)) != cudaSuccess)
         return e;
-    if ((e = cudaStreamSynchronize(p.stream)) != cudaSuccess)
-        return e;
-    out.iters += p.cg_info_host[0];
-    p.ctr.cg_iters += p.cg_info_host[0];
+    const char *what = sizeof(TV) == 8 ? "bond fp64" : "bond fp32";
+    if constexpr (sizeof(TV) == 8)
     {
-        float ms = 0;
-        if (cudaEventElapsedTime(&ms, p.cg_ev[0], p.cg_ev[1]) == cudaSuccess)
-            p.ctr.cg_kernel_seconds += ms * 1e-3;
-        static const bool log = std::getenv("LPMGPU_LOG") != nullptr;
-        if (log)
-            std::fprintf(stderr, "lpmgpu cg launch %lld: %s%s iters=%lld ms=%.3f grid=%d\n",
-                         (long long)p.ctr.cg_launches, sizeof(TK) == 8 ? "fp64" : "fp32", D == 2 ? "/2d" : "/3d",
-                         (long long)p.cg_info_host[0], ms, grid);
+        if (bond_cluster_fits(p))
+        {
+            what = "bond fp64 cluster";
+            e = enqueue_bond_cluster(p, b, x, rtol, atol, abs_stop, maxit);
+        }
+        else
+            e = enqueue_bond_grid<TV>(p, b, x, r, pa, pb, rtol, atol, abs_stop, maxit);
     }
-    if (p.cg_info_host[1] & 1)
-        out.maxit_hits++;
-    if (p.cg_info_host[1] & 2)
-        out.timeout = true;
-    if (p.cg_info_host[1] & 4)
-        out.breakdown = true;
-    if (rr_final)
-        *rr_final = reinterpret_cast<double *>(p.cg_info_host)[3];
-    return cudaSuccess;
+    else
+        e = enqueue_bond_grid<TV>(p, b, x, r, pa, pb, rtol, atol, abs_stop, maxit);
+    if (e != cudaSuccess)
+        return e;
+    return finish_cg(p, what, out, rr_final, declined);
 }
 
 template <int D>
@@ -439,6 +479,19 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
 {
     const int64_t ndof = (int64_t)p.n * D;
     const int64_t maxit = p.desc.cg_maxit > 0 ? p.desc.cg_maxit : ndof;
+    bool declined = false;
+    if (p.bo_valid && (p.desc.precision != LPMGPU_MIXED || bond_cluster_fits(p)))
+    {
+        // Mixed precision in the cluster form: its bonds are in shared memory and its iterations are
+        // bound by latency, not by bytes, so the correction is solved for in FP64 at once.
+        const cudaError_t e = run_bond<double>(p, p.res, p.x, p.r, p.p0, p.p1, p.desc.cg_rtol, p.desc.cg_atol, -1.0,
+                                               maxit, out, nullptr, &declined);
+        if (e != cudaSuccess || !declined)
+        {
+            out.refinements += p.desc.precision == LPMGPU_MIXED ? 1 : 0;
+            return e;
+        }
+    }
     if (p.desc.precision != LPMGPU_MIXED)
         return run_cg<double, double, D>(p, p.K, p.res, p.x, p.r, p.p0, p.p1, p.q, p.desc.cg_rtol, p.desc.cg_atol,
                                          -1.0, maxit, out, nullptr);
@@ -459,6 +512,7 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
         return e;
     const double stop = p.desc.cg_rtol * rr0 + p.desc.cg_atol;
     rr = rr0;
+    bool bond = p.bo_valid && !declined;
     for (int ref = 0; ref < 30 && !(rr <= stop); ++ref)
     {
         if ((e = enqueue_r_to_b32(p)) != cudaSuccess)
@@ -466,7 +520,12 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
         // the inner solve aims a little below the outer target, measured on its own residual
         CGResult inner;
         double rr_in = 0;
-        if ((e = run_cg<float, float, D>(p, p.K32, p.b32, p.x32, p.r32, p.pa32, p.pb32, p.q32, 0.0, 0.0, 0.25 * stop,
+        bool off = !bond;
+        if (bond && (e = run_bond<float>(p, p.b32, p.x32, p.r32, p.pa32, p.pb32, 0.0, 0.0, 0.25 * stop, maxit, inner,
+                                         &rr_in, &off)) != cudaSuccess)
+            return e;
+        bond = !off;
+        if (off && (e = run_cg<float, float, D>(p, p.K32, p.b32, p.x32, p.r32, p.pa32, p.pb32, p.q32, 0.0, 0.0, 0.25 * stop,
                                          maxit, inner, &rr_in)) != cudaSuccess)
             return e;
         out.iters += inner.iters;
@@ -561,13 +620,42 @@ cudaError_t solve_linear(Problem &p, CGResult &out)
 // the barriers dominate and fewer, fuller blocks can be faster.  The tuner times `iterations` CG
 // iterations of this problem's own matrix for each candidate grid (the default and its 3/4, 1/2,
 // 1/4, 1/8, 1/16), twice each, and keeps the fastest by its second timing.  Candidates are never
-// above the default, so every one is co-resident.
+// above the default, so every one is co-resident.  For a problem that runs in one cluster the grid is
+// the cluster's CTAs (rounded down to a power of two that still holds the problem).
 template <typename TK, typename TV, int D>
 static cudaError_t tune_dim(Problem &p, int iterations, lpmgpu_tune_result *res, const TK *K, const TV *b, TV *x,
                             TV *r, TV *pa, TV *pb, TV *q)
 {
     int g0 = 0;
-    cudaError_t e = cg_grid_rule<TK, TV, D>(p, &g0);
+    const int saved = p.cg_grid;
+    p.cg_grid = 0;
+    bool bond = p.bo_valid;
+    const bool cluster = bond && bond_cluster_fits(p);
+    // the solve that solve_dim runs: the bond form (FP64 in one cluster whatever the precision), or the
+    // assembled matrix for a K without one
+    auto solve = [&](CGResult &cr) -> cudaError_t {
+        bool off = !bond;
+        cudaError_t e2 = cudaSuccess;
+        if (bond && cluster)
+            e2 = run_bond<double>(p, p.diag_raw, p.x, p.r, p.p0, p.p1, 0.0, 0.0, 0.0, iterations, cr, nullptr, &off);
+        else if (bond)
+            e2 = run_bond<TV>(p, b, x, r, pa, pb, 0.0, 0.0, 0.0, iterations, cr, nullptr, &off);
+        if (e2 == cudaSuccess && off)
+            e2 = run_cg<TK, TV, D>(p, K, b, x, r, pa, pb, q, 0.0, 0.0, 0.0, iterations, cr, nullptr);
+        return e2;
+    };
+    cudaError_t e = cudaSuccess;
+    if (bond)
+    { // whether this K has a bond form is known once a launch has looked at its flags
+        int flag = 0;
+        e = cudaMemcpyAsync(&flag, &p.scal->bond_flag, sizeof(int), cudaMemcpyDeviceToHost, p.stream);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(p.stream);
+        bond = (flag & bond_flags_bad(p)) == 0;
+    }
+    if (e == cudaSuccess)
+        e = bond ? bond_default_grid<TV>(p, &g0) : cg_grid_rule<TK, TV, D>(p, &g0);
+    p.cg_grid = saved;
     if (e != cudaSuccess)
         return e;
     std::vector<int> cand;
@@ -577,7 +665,6 @@ static cudaError_t tune_dim(Problem &p, int iterations, lpmgpu_tune_result *res,
         if (std::find(cand.begin(), cand.end(), g) == cand.end() && (int)cand.size() < LPMGPU_TUNE_MAX)
             cand.push_back(g);
     }
-    const int saved = p.cg_grid;
     const lpmgpu_counters ctr = p.ctr;
     int best = g0;
     double best_us = 0;
@@ -589,7 +676,7 @@ static cudaError_t tune_dim(Problem &p, int iterations, lpmgpu_tune_result *res,
         for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep)
         {
             CGResult cr;
-            e = run_cg<TK, TV, D>(p, K, b, x, r, pa, pb, q, 0.0, 0.0, 0.0, iterations, cr, nullptr);
+            e = solve(cr);
             float ms = 0;
             if (e == cudaSuccess && (e = cudaEventElapsedTime(&ms, p.cg_ev[0], p.cg_ev[1])) == cudaSuccess)
                 us = cr.iters > 0 ? 1e3 * ms / (double)cr.iters : 0.0;

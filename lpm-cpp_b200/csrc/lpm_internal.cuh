@@ -46,7 +46,8 @@ struct Scalars
     double pad;
     int any_flag;         // damage update: some bond broke / damage changed
     int err;              // topology overflow or a timed-out wait
-    int pad2[2];
+    int bond_flag;        // of the K assembled last: why the bond form cannot serve it (bond_op.cuh)
+    int pad2;
 };
 
 // Device state of one problem.  Particles are indexed by id; bonds are owner-major CSR
@@ -150,6 +151,17 @@ struct Problem
     int64_t *asm_row = nullptr;
     int *asm_pb = nullptr, *asm_asym = nullptr;
     int64_t asm_paths = 0;
+    // bond form of K (bond_op.cuh): its layout, this assembly's cosines and coefficients, and theta
+    bool bo_ok = false;         // the layout exists
+    bool bo_valid = false;      // it holds the K assembled last
+    bool bo_gen = false;        // coefficients per bond (the general form)
+    int bo_ls = 0, bo_ng = 0, bo_width = 0, bo_nc = 0;
+    int *bo_col = nullptr, *bo_src = nullptr;
+    int *bo_reach = nullptr;
+    std::vector<int> bo_reach_host;
+    unsigned char *bo_mask = nullptr;
+    double *bo_c = nullptr, *bo_tm = nullptr, *bo_row = nullptr, *bo_th = nullptr;
+    float *bo_c32 = nullptr, *bo_tm32 = nullptr, *bo_row32 = nullptr, *bo_th32 = nullptr;
 };
 
 constexpr int kMaxGridBlocks = 4096;
@@ -174,6 +186,18 @@ cudaError_t prim_max(cudaStream_t st, const int *in, int64_t count, int *dev_out
 cudaError_t prim_sort_pairs(cudaStream_t st, const int *key, const int *val, int *skey, int *sval, int64_t n);
 // each segment [off[s], off[s+1]) of non-negative values sorted ascending, in -> out
 cudaError_t prim_segmented_sort(cudaStream_t st, const int *in, int *out, int64_t total, int nseg, const int *off);
+// the bond form of K and the CG on it (bond_op.cu)
+cudaError_t setup_bond_op(Problem &p);
+cudaError_t launch_bond_refresh(Problem &p, bool apply_bc);
+bool bond_cluster_fits(const Problem &p); // K as assembled last has a bond form that fits one cluster
+int bond_flags_bad(const Problem &p);      // the bits of Scalars::bond_flag that rule the bond form out
+cudaError_t enqueue_bond_cluster(Problem &p, const double *b, double *x, double rtol, double atol, double abs_stop,
+                                 int64_t maxit);
+template <typename TV>
+cudaError_t enqueue_bond_grid(Problem &p, const TV *b, TV *x, TV *r, TV *pa, TV *pb, double rtol, double atol,
+                              double abs_stop, int64_t maxit);
+template <typename TV>
+cudaError_t bond_default_grid(const Problem &p, int *grid);
 cudaError_t launch_update_state_var(Problem &p);
 cudaError_t launch_static_damage(Problem &p);   // sets p.scal->any_flag
 // nonlocal damage (damage.cu): the neighbour search at creation, the averaged damage rate,

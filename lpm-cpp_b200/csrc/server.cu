@@ -105,6 +105,11 @@ int64_t estimate_bytes(const lpmgpu_desc &d)
     // the fast assembly's lists: at most nb^2 two-hop paths of 5 bytes, a count per slot, T and
     // Ts per bond, U and the row offset per particle
     per_particle += (int64_t)nb * nb * 5 + nc + (int64_t)nb * 16 + 56;
+    // the bond form of K: per bond (rows padded to the lanes that share them) a column, its source
+    // bond, the cosines and two coefficients; per particle theta, S, U, the self block and a mask
+    per_particle += (int64_t)(nb + 8) * (24 + 8 * dim) + 192;
+    if (d.precision == LPMGPU_MIXED)
+        per_particle += (int64_t)(nb + 8) * (8 + 4 * dim) + 96;
     if (d.nonlocal_cutoff_ratio > 0 && d.radius > 0)
     {
         // nonlocal lists: the particles within cutoff_ratio x nonlocal_L, counted for the densest

@@ -135,6 +135,10 @@ cudaError_t enqueue_assemble(Problem &p, bool apply_bc)
     cudaError_t e = launch_assemble(p, apply_bc, mixed ? &k32 : nullptr);
     if (e == cudaSuccess && mixed && !k32)
         e = launch_k_to_f32(p);
+    // the bit-exact kernel's K is solved as assembled
+    p.bo_valid = p.bo_ok && p.asm_fast && !p.asm_exact;
+    if (e == cudaSuccess && p.bo_valid)
+        e = launch_bond_refresh(p, apply_bc);
     return e;
 }
 
@@ -676,6 +680,23 @@ static void free_problem(Problem &p)
         cudaStreamDestroy(p.stream);
 }
 
+// Whether the description's per-bond arrays (if any) hold just what setParticleProperty gives every
+// bond of a layer (k_bonds_fill): the C++ drop-ins pass them for every Assembly.
+static bool uniform_bonds(const Problem &p, const lpmgpu_desc &d)
+{
+    const bool hex = p.cell.lattice == LPMGPU_HEXAGON2D;
+    const double kn[2] = {p.kntv[0], hex ? p.kntv[0] : p.kntv[1]}, tv = hex ? p.kntv[1] : p.kntv[2];
+    if (!d.bond_kn && !d.bond_tv && !d.bond_damage)
+        return true;
+    size_t b = 0;
+    for (int i = 0; i < d.n; ++i)
+        for (int q = 0; q < d.bond_nb0[i] + d.bond_nb1[i]; ++q, ++b)
+            if ((d.bond_kn && d.bond_kn[b] != kn[q < d.bond_nb0[i] ? 0 : 1]) || (d.bond_tv && d.bond_tv[b] != tv) ||
+                (d.bond_damage && d.bond_damage[b] != 0.0 && d.bond_damage[b] != 1.0))
+                return false;
+    return true;
+}
+
 int32_t lpmgpu_create(const lpmgpu_desc *d, lpmgpu_solver **out)
 {
     if (!d || !out || !d->xyz || d->n <= 0 || d->lattice < 0 || d->lattice > LPMGPU_BCC3D ||
@@ -810,6 +831,7 @@ int32_t lpmgpu_create(const lpmgpu_desc *d, lpmgpu_solver **out)
         set_last_error("a particle has no bonds, or more bonds / connections than supported");
         return fail(topo_err);
     }
+    p.bo_gen = !uniform_bonds(p, *d);
     const size_t ndof = n * p.dim;
     CKF(dalloc(p, &p.K, (size_t)p.nsb * p.dim * p.dim * kSlice));
     CKF(dalloc(p, &p.diag_raw, ndof));
@@ -833,7 +855,10 @@ int32_t lpmgpu_create(const lpmgpu_desc *d, lpmgpu_solver **out)
         CKF(dalloc(p, &p.s32b, ndof));
     }
     if (!std::getenv("LPMGPU_ASSEMBLY_EXACT"))
+    {
         CKF(setup_fast_assembly(p));
+        CKF(setup_bond_op(p));
+    }
     // the examples run updateGeometry + updateForceState before constructing the solver
     CKF(launch_geometry_force(p));
     CKF(launch_update_rr_impl(p, false));
