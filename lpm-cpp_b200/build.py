@@ -20,7 +20,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # sources compiled with FMA contraction: the fast assembly, whose results are held to the
 # reference within rounding instead of bit for bit, and the batched CG, whose members are held to
 # their twins solved alone within tolerances (its partition already orders the sums differently)
-CONTRACTED = {"assembly_fast.cu", "batch.cu", "bond_op.cu"}
+CONTRACTED = {"assembly_fast.cu", "batch.cu", "bond_op.cu", "direct.cu"}
 
 
 def nvcc() -> str:

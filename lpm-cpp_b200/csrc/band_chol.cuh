@@ -8,10 +8,8 @@
 //
 // The factorisation is blocked in column blocks [j0, j0 + jb): the diagonal block is factored,
 // the rows below it in the band are solved against it (L21 = A21 L11^-T), and the trailing band
-// window is updated (A22 -= L21 L21^T).  Each function below is the whole work of one thread of
-// one kernel, and the threads of a kernel never touch one another's outputs, so the kernels are
-// race-free and a host loop over the same thread indices computes the same bits.  Every function
-// compiles as device and as host code: the tests run this exact code on the CPU.
+// window is updated (A22 -= L21 L21^T).  The functions below state that algorithm entry by entry; the
+// host tests run them, and the device (direct.cu) takes the same sums in tiles.
 #pragma once
 
 #include <cmath>

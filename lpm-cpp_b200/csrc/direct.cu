@@ -8,9 +8,10 @@
 //   * Band fill (device): the BC-eliminated stiffness, read from its sliced-ELL blocks, into the
 //     permuted lower band (band_chol.cuh's layout).
 //   * Factorisation (device, once per assembled K: K is fixed through a load step's Newton
-//     iterations, solver_static.h:107-118): blocked band Cholesky in column blocks of kBandNB,
-//     three kernels per block (diagonal block, rows below it, trailing window).
-//   * Solve (device, every Newton iteration): forward and backward substitution on the factor.
+//     iterations, solver_static.h:107-118): blocked band Cholesky in column blocks of kBandNB in
+//     one persistent launch.
+//   * Solve (device, every Newton iteration): forward and backward substitution on the factor, in
+//     one CTA.
 // The band costs n * (kd + 1) doubles; 2D plates fit easily, wide 3D bands are rejected with
 // LPMGPU_ERR_OUT_OF_MEMORY before anything is allocated.  A pivot that is not positive (a
 // singular or indefinite K, e.g. a particle left without bonds) is LPMGPU_ERR_NOT_SPD.
@@ -20,7 +21,7 @@
 #include <vector>
 
 #include "band_chol.cuh"
-#include "lpm_internal.cuh"
+#include "cg_device.cuh"
 
 namespace lpm
 {
@@ -138,129 +139,456 @@ __global__ void k_band_fill(int n, const int *__restrict__ rowptr, const int *__
     }
 }
 
-// The diagonal block by one warp: the block's lower triangle (inside the band) staged in shared
-// memory, lane i owning row i.  Per column jj: the pivot's square root, the column scaled, the
-// trailing entries updated, each entry receiving exactly the operations, in the order, of
-// band::potrf_block (which the host tests run), so the factor is bit for bit the same.
-__global__ void __launch_bounds__(32) k_potrf(double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb, int *fail)
-{
-    __shared__ double a[32][33];
-    __shared__ int bad;
-    const int i = threadIdx.x;
-    if (i == 0)
-        bad = 0;
-    if (i < jb)
-        for (int j = 0; j <= i; ++j)
-            a[i][j] = (i - j <= kd) ? band::at(AB, ldab, j0 + i, j0 + j) : 0.0;
-    __syncwarp();
-    for (int jj = 0; jj < jb; ++jj)
-    {
-        if (i == jj)
-        {
-            const double v = a[jj][jj];
-            if (!(v > 0.0))
-                bad = jj + 1;
-            else
-                a[jj][jj] = sqrt(v);
-        }
-        __syncwarp();
-        if (bad)
-            break;
-        const double d = a[jj][jj];
-        if (i > jj && i < jb && i - jj <= kd)
-            a[i][jj] = a[i][jj] / d;
-        __syncwarp();
-        // row i: entries (i, c), jj < c <= i, in ascending c as the one-thread loop reaches them
-        if (i > jj && i < jb && i - jj <= kd)
-            for (int c = jj + 1; c <= i; ++c)
-                if (c - jj <= kd)
-                    a[i][c] = a[i][c] - a[i][jj] * a[c][jj];
-        __syncwarp();
-    }
-    if (bad)
-    {
-        if (i == 0 && *fail == 0)
-            *fail = (int)(j0 + bad);
-        return;
-    }
-    if (i < jb)
-        for (int j = 0; j <= i; ++j)
-            if (i - j <= kd)
-                band::at(AB, ldab, j0 + i, j0 + j) = a[i][j];
-}
+// ---- factorisation: one persistent launch
+//
+// Per 32-column block: the rows below are solved against the factored block (four rows per warp), and
+// after a barrier the trailing window is updated with FP64 tensor instructions (the update is a product
+// of two panels) while warp 0 of every CTA updates and factors the next diagonal block (repeating it
+// costs less than another exchange); a second barrier ends the block.  Bound by the diagonal blocks'
+// serial pivots, then by the latency of the window's entries and two grid barriers (2.5 us each).
+// Factor and solve of the 50 x 58 hexagonal plate (5,800 unknowns, half-bandwidth 401) 46.0 -> 3.7 ms,
+// 100 x 115 (23,000, 801) 330 -> 19.3 ms, against three launches per block and one warp per diagonal
+// block.  One 16-CTA cluster, whose barrier takes 0.3 us, took 4.0 and 33.1 ms: its SMs hold too few
+// window tiles in flight.
+constexpr int kFactorThreads = 256;
+constexpr int kFactorWarps = kFactorThreads / 32;
 
-// The rows below the diagonal block, one thread per row, with the factored block and the thread's
-// row staged in shared memory; each entry gets band::trsm_row's operations in its order.
-constexpr int kTrsmThreads = 128;
-__global__ void __launch_bounds__(kTrsmThreads) k_trsm(double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb,
-                                                       int64_t m2)
+// All blocks of the cooperative launch: a counting barrier in global memory (bounded: false and
+// *fail = -1 once a wait passed the limit).
+__device__ __forceinline__ bool factor_barrier(unsigned *bar, unsigned &epoch, int *fail, int *s_stop)
 {
-    __shared__ double L[32][33];
-    __shared__ double row[kTrsmThreads][33];
-    for (int q = threadIdx.x; q < 32 * 32; q += blockDim.x)
-    {
-        const int r = q / 32, c = q % 32;
-        L[r][c] = (r < jb && c <= r && r - c <= kd) ? band::at(AB, ldab, j0 + r, j0 + c) : 0.0;
-    }
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t i = j0 + jb + t;
-    double *w = row[threadIdx.x];
-    if (t < m2)
-        for (int jj = 0; jj < jb; ++jj)
-            w[jj] = (i - (j0 + jj) <= kd) ? band::at(AB, ldab, i, j0 + jj) : 0.0;
     __syncthreads();
-    if (t >= m2)
-        return;
-    for (int jj = 0; jj < jb; ++jj)
+    if (threadIdx.x == 0)
     {
-        const int64_t j = j0 + jj;
-        if (i - j > kd)
-            continue;
-        double v = w[jj];
-        for (int kk = 0; kk < jj; ++kk)
-            if (i - (j0 + kk) <= kd)
-                v = v - w[kk] * L[jj][kk];
-        v = v / L[jj][jj];
-        w[jj] = v;
-        band::at(AB, ldab, i, j) = v;
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const unsigned target = (epoch + 1u) * gridDim.x;
+        const unsigned long long t0 = gtimer();
+        while ((int)(ld_acquire(bar) - target) < 0)
+            if (gtimer() - t0 > kBarrierTimeoutNs)
+            {
+                atomicExch(fail, -1);
+                *s_stop = 1;
+                break;
+            }
+    }
+    epoch++;
+    __syncthreads();
+    return *s_stop == 0;
+}
+
+// D += A B^T for 8 x 4 panels: lane l holds row l / 4, column l % 4 of each operand and the entries
+// (l / 4, 2 (l % 4)) and the next one of D
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+// The factor of a 32 x 32 block by one warp: lane i holds row i in v and gets the pivots in fours, after
+// which its row moves down by four columns (straight-line code for all 32 would not fit the instruction
+// caches, and every block runs it once).  Column j goes to L[j][.] (zero above the diagonal and behind
+// row 31), the reciprocal of its diagonal to inv[j].  Returns 0, or 1 + the column of a pivot that is
+// not positive.
+constexpr int kLRow = 66; // doubles per column of L: 32 rows, 32 zeros, 2 to shift the banks
+__device__ __forceinline__ int factor_block(double *v, double (*L)[kLRow], double *inv)
+{
+    const int lane = threadIdx.x & 31;
+    int bad = 0;
+    double d = __shfl_sync(0xffffffffu, v[0], 0);
+#pragma unroll 1
+    for (int j4 = 0; j4 < 32; j4 += 4)
+    {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int j = j4 + u;
+            if (bad == 0 && !(d > 0.0))
+                bad = j + 1;
+            const double is = rsqrt(d);
+            v[u] *= is; // lane j: d / sqrt(d)
+            // the next pivot is ready in its own lane before the column's other updates
+            d = __shfl_sync(0xffffffffu, v[u + 1] - v[u] * v[u], (j + 1) & 31);
+            L[j][lane] = lane >= j ? v[u] : 0.0;
+            if (lane == j)
+                inv[j] = is;
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 32; c += 2)
+                if (c + 1 > u)
+                {
+                    const double2 w = *reinterpret_cast<const double2 *>(&L[j][j4 + c]);
+                    if (c > u)
+                        v[c] -= v[u] * w.x;
+                    v[c + 1] -= v[u] * w.y;
+                }
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            v[c] = c < 28 ? v[c < 28 ? c + 4 : 31] : 0.0;
+    }
+    return bad;
+}
+
+__global__ void __launch_bounds__(kFactorThreads, 1) k_band_factor(double *AB, int64_t ldab, int64_t kd, int64_t n,
+                                                                  int *fail, unsigned *bar)
+{
+    extern __shared__ __align__(16) unsigned char fsm[];
+    double(*Lb)[32][kLRow] = reinterpret_cast<double(*)[32][kLRow]>(fsm); // this block's factor and the next one's
+    double(*T)[33] = reinterpret_cast<double(*)[33]>(fsm + 2 * sizeof(double) * 32 * kLRow);
+    __shared__ double inv[2][32];
+    __shared__ int bad, s_stop;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t gw = (int64_t)blockIdx.x * kFactorWarps + warp, nwarps = (int64_t)kFactorWarps * gridDim.x;
+    const int r8 = lane >> 2, k4 = lane & 3;
+    unsigned epoch = 0;
+    if (threadIdx.x == 0)
+        s_stop = bad = 0;
+    for (int k = threadIdx.x; k < 2 * 32 * kLRow; k += blockDim.x)
+        (&Lb[0][0][0])[k] = 0.0;
+    __syncthreads();
+    if (warp == 0) // the first block: lane i reads row i; a missing row or column is the identity's
+    {
+        const int jb = (int)min((int64_t)kBandNB, n);
+        double v[33];
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            v[j] = (lane < jb && j <= lane && lane - j <= kd) ? AB[(lane - j) + j * ldab] : (j == lane && lane >= jb) ? 1.0 : 0.0;
+        v[32] = 0.0;
+        const int b = factor_block(v, Lb[0], inv[0]);
+        if (lane == 0)
+            bad = b;
+    }
+    __syncthreads();
+    for (int64_t j0 = 0; j0 < n; j0 += kBandNB)
+    {
+        const int cur = (int)((j0 / kBandNB) & 1);
+        const int jb = (int)min((int64_t)kBandNB, n - j0);
+        const int64_t c0 = j0 + jb, end = band::below_end(n, kd, j0, jb), m2 = end - c0;
+        if (bad)
+        {
+            if (blockIdx.x == 0 && threadIdx.x == 0)
+                *fail = (int)(j0 + bad);
+            return; // every CTA factored the same block
+        }
+        // the rows below against the factored block: four rows per warp, a lane per column
+        const double(*L)[kLRow] = Lb[cur];
+        for (int64_t q = gw; 4 * q < m2; q += nwarps)
+        {
+            const int64_t i0 = c0 + 4 * q;
+            double *const col = AB + (j0 + lane) * ldab - (j0 + lane); // entry (i, j0 + lane) at col[i]
+            double x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                x[u] = (i0 + u < end && lane < jb && i0 + u - (j0 + lane) <= kd) ? col[i0 + u] : 0.0;
+#pragma unroll 4
+            for (int j = 0; j < 32; ++j)
+            {
+                const double l = lane > j ? L[j][lane] : 0.0, ij = inv[cur][j];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const double y = __shfl_sync(0xffffffffu, x[u], j) * ij;
+                    x[u] = lane == j ? y : x[u] - y * l;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u < end && lane < jb && i0 + u - (j0 + lane) <= kd)
+                    col[i0 + u] = x[u];
+        }
+        if (!factor_barrier(bar, epoch, fail, &s_stop))
+            return;
+        // the factor takes the block's place (every CTA has long read it)
+        if (blockIdx.x == gridDim.x - 1 && warp == kFactorWarps - 1 && lane < jb)
+            for (int j = 0; j <= lane; ++j)
+                if (lane - j <= kd)
+                    AB[(lane - j) + (j0 + j) * ldab] = L[j][lane];
+        if (m2 <= 0)
+            break; // the last block
+        if (warp == 0)
+        {
+            // the next diagonal block: this block's update of it, then its factor, in every CTA
+            const int nb = (int)min((int64_t)kBandNB, n - c0);
+            double d[4][4][2];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; ++y)
+                    d[x][y][0] = d[x][y][1] = 0.0;
+            double v[33];
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                v[j] = (lane < nb && j <= lane && lane - j <= kd) ? AB[(lane - j) + (c0 + j) * ldab]
+                       : (j == lane && lane >= nb)                ? 1.0
+                                                                  : 0.0;
+            v[32] = 0.0;
+#pragma unroll
+            for (int k = 0; k < kBandNB; k += 4)
+            {
+                const int64_t j = j0 + k + k4;
+                const double *col = AB + j * ldab - j;
+                double a[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                {
+                    const int64_t i = c0 + 8 * x + r8;
+                    a[x] = (i < end && i - j <= kd) ? col[i] : 0.0;
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y <= x; ++y)
+                        dmma(d[x][y][0], d[x][y][1], a[x], a[y]);
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y <= x; ++y)
+                {
+                    T[8 * x + r8][8 * y + 2 * k4] = d[x][y][0];
+                    T[8 * x + r8][8 * y + 2 * k4 + 1] = d[x][y][1];
+                }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (j <= lane)
+                    v[j] -= T[lane][j];
+            __syncwarp();
+            const int b = factor_block(v, Lb[cur ^ 1], inv[cur ^ 1]);
+            if (lane == 0)
+                bad = b;
+        }
+        else
+        {
+            // trailing window below the next diagonal block, in tiles of 32 x 16, a warp each:
+            // A(i, c) -= sum_k L(i, k) L(c, k)
+            const int64_t tr = (m2 + 31) / 32, tc = (m2 + 15) / 16;
+            const int64_t first = (int64_t)(warp - 1) * gridDim.x + blockIdx.x, step = (int64_t)(kFactorWarps - 1) * gridDim.x;
+            for (int64_t t = first; t < (tr - 1) * tc; t += step)
+            {
+                const int64_t ti = 1 + t / tc, tj = t % tc, i0 = c0 + ti * 32, cc = c0 + tj * 16;
+                if (cc > i0 + 31 || i0 - (cc + 15) > kd)
+                    continue; // above the diagonal, or outside the band
+                double d[4][2][2], w[4][2][2]; // the product; the window's entries, on their way meanwhile
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                        {
+                            const int64_t i = i0 + 8 * x + r8, c = cc + 8 * y + 2 * k4 + e;
+                            d[x][y][e] = 0.0;
+                            w[x][y][e] = (c <= i && i < end && i - c <= kd) ? AB[(i - c) + c * ldab] : 0.0;
+                        }
+#pragma unroll
+                for (int k = 0; k < kBandNB; k += 4) // rows below exist: the block has all its columns
+                {
+                    const int64_t j = j0 + k + k4;
+                    const double *col = AB + j * ldab - j; // entry (i, j) at col[i]
+                    double a[4], b[2];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                    {
+                        const int64_t i = i0 + 8 * x + r8;
+                        a[x] = (i < end && i - j <= kd) ? col[i] : 0.0;
+                    }
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+                    {
+                        const int64_t i = cc + 8 * y + r8;
+                        b[y] = (i < end && i - j <= kd) ? col[i] : 0.0;
+                    }
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+#pragma unroll
+                        for (int y = 0; y < 2; ++y)
+                            dmma(d[x][y][0], d[x][y][1], a[x], b[y]);
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                        {
+                            const int64_t i = i0 + 8 * x + r8, c = cc + 8 * y + 2 * k4 + e;
+                            if (c <= i && i < end && i - c <= kd)
+                                AB[(i - c) + c * ldab] = w[x][y][e] - d[x][y][e];
+                        }
+            }
+        }
+        if (!factor_barrier(bar, epoch, fail, &s_stop))
+            return;
     }
 }
 
-// threads along i (contiguous band columns), blocks along c
-__global__ void k_syrk(double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb, int64_t m2)
+constexpr int kFactorSmem = 2 * 8 * 32 * kLRow + 8 * 32 * 33;
+
+// ---- substitution: one CTA
+//
+// Forward, block by block: one warp solves the block's triangle (lane i holds y_i), then the rows
+// below take their 32 products.  Backward: a warp per column of the block
+// gathers the finished x below it, then one warp solves the transposed triangle.  Bound by the chain
+// of 32 pivots per block, so more CTAs would only add barriers.  Both sweeps over 5,800 unknowns at
+// half-bandwidth 401: 1.15 ms (2.74 ms without the panels; 25 ms with four launches per block).
+constexpr int kSolveThreads = 1024;
+constexpr int kSolvePanelBytes = 104 * 1024; // one panel; two are in shared memory
+static_assert(2 * kSolvePanelBytes + 12 * 1024 <= 232448, "shared memory of the substitution");
+
+// `panel` holds a block's 32 whole band columns (one contiguous piece of the band) when they fit,
+// copied there ahead of their use; wider bands are read from global memory.
+template <bool PANEL>
+__global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *AB, int64_t ldab, int64_t kd, int64_t n,
+                                                                double *y)
 {
-    const int64_t c0 = j0 + jb, e = c0 + m2;
-    for (int64_t cy = blockIdx.y; cy < m2; cy += gridDim.y)
+    extern __shared__ __align__(128) unsigned char dsm[];
+    __shared__ double M[32][33]; // M[j][i]: column j, row i of the block, over the diagonal entry j
+    __shared__ double inv[32], s[32];
+    __shared__ int lost; // a copy did not arrive in time
+    __shared__ __align__(8) unsigned long long bar[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t nblk = (n + kBandNB - 1) / kBandNB;
+    if (threadIdx.x == 0)
     {
-        const int64_t c = c0 + cy;
-        const int64_t i = c + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < e && i - c <= kd)
-            band::syrk_entry(AB, ldab, kd, j0, jb, i, c);
+        lost = 0;
+        for (int k = 0; k < 2; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&bar[k])) : "memory");
     }
-}
-
-__global__ void k_fwd_block(const double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb, double *y)
-{
-    band::fwd_block(AB, ldab, kd, j0, jb, y);
-}
-
-__global__ void k_fwd_update(const double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb, int64_t m2, double *y)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < m2)
-        band::fwd_update_row(AB, ldab, kd, j0, jb, j0 + jb + t, y);
-}
-
-__global__ void k_bwd_update(const double *AB, int64_t ldab, int64_t kd, int64_t n, int64_t j0, int64_t jb, double *y)
-{
-    const int64_t t = threadIdx.x;
-    if (t < jb)
-        band::bwd_update_col(AB, ldab, kd, n, j0, jb, j0 + t, y);
-}
-
-__global__ void k_bwd_block(const double *AB, int64_t ldab, int64_t kd, int64_t j0, int64_t jb, double *y)
-{
-    band::bwd_block(AB, ldab, kd, j0, jb, y);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    // the copies run through blocks 0 .. nblk - 1, then back to 0; copy q goes to buffer q % 2
+    auto block_of = [&](int64_t q) { return q < nblk ? q : 2 * nblk - 1 - q; };
+    auto fetch = [&](int64_t q) {
+        if (!PANEL || threadIdx.x != 0 || q >= 2 * nblk)
+            return;
+        const int64_t j0 = block_of(q) * kBandNB, jb = min((int64_t)kBandNB, n - j0);
+        // whole 16-byte pieces; the allocation has one spare entry behind an odd last column
+        const unsigned bytes = (unsigned)((jb * ldab * 8 + 15) / 16 * 16);
+        const unsigned b = (unsigned)__cvta_generic_to_shared(&bar[q & 1]);
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(dsm + (q & 1) * kSolvePanelBytes);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                     "l"(AB + j0 * ldab), "r"(bytes), "r"(b)
+                     : "memory");
+    };
+    // column j of block q, entry (i, j) at [i - j]
+    auto column = [&](int64_t q, int64_t j0, int j) -> const double * {
+        return PANEL ? reinterpret_cast<const double *>(dsm + (q & 1) * kSolvePanelBytes) + j * ldab
+                     : AB + (j0 + j) * ldab;
+    };
+    auto arrive = [&](int64_t q) {
+        if (!PANEL)
+            return;
+        const unsigned b = (unsigned)__cvta_generic_to_shared(&bar[q & 1]), parity = (unsigned)((q >> 1) & 1);
+        const unsigned long long t0 = gtimer();
+        unsigned done = 0;
+        while (!done && gtimer() - t0 < kBarrierTimeoutNs)
+            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                         : "=r"(done)
+                         : "r"(b), "r"(parity)
+                         : "memory");
+        if (!done)
+            lost = 1;
+    };
+    auto stage = [&](int64_t q, int64_t j0, int jb, bool transposed) { // warp w: column w
+        const double v = (warp < jb && lane < jb && lane >= warp && lane - warp <= kd) ? column(q, j0, warp)[lane - warp]
+                                                                                        : (lane == warp ? 1.0 : 0.0);
+        const double dj = 1.0 / __shfl_sync(0xffffffffu, v, warp);
+        if (lane == warp)
+            inv[warp] = dj;
+        // forward: column j over its diagonal; backward: row i of L^T over the diagonal of i, which
+        // column j's thread i learns from the other warps' diagonals
+        if (!transposed)
+            M[warp][lane] = v * dj;
+        else
+            M[lane][warp] = v;
+    };
+    fetch(0);
+    fetch(1);
+    for (int64_t q = 0; q < nblk; ++q)
+    {
+        const int64_t j0 = q * kBandNB;
+        const int jb = (int)min((int64_t)kBandNB, n - j0);
+        const int64_t c0 = j0 + jb, end = band::below_end(n, kd, j0, jb);
+        arrive(q);
+        stage(q, j0, jb, false);
+        __syncthreads();
+        if (warp == 0)
+        {
+            double v = lane < jb ? y[j0 + lane] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+            {
+                const double x = __shfl_sync(0xffffffffu, v, j);
+                v -= lane > j ? M[j][lane] * x : 0.0;
+            }
+            v *= inv[lane];
+            s[lane] = v;
+            if (lane < jb)
+                y[j0 + lane] = v;
+        }
+        __syncthreads();
+        for (int64_t i = c0 + threadIdx.x; i < end; i += blockDim.x)
+        {
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 8
+            for (int j = 0; j < jb; ++j)
+                if (i - (j0 + j) <= kd)
+                    t[j & 3] += column(q, j0, j)[i - j0 - j] * s[j];
+            y[i] -= (t[0] + t[1]) + (t[2] + t[3]);
+        }
+        __syncthreads();
+        fetch(q + 2);
+    }
+    for (int64_t q = nblk; q < 2 * nblk; ++q)
+    {
+        const int64_t j0 = block_of(q) * kBandNB;
+        const int jb = (int)min((int64_t)kBandNB, n - j0);
+        const int64_t c0 = j0 + jb, end = band::below_end(n, kd, j0, jb);
+        arrive(q);
+        stage(q, j0, jb, true);
+        if (warp < jb)
+        {
+            const int64_t j = j0 + warp;
+            const double *col = column(q, j0, warp) - j; // entry (i, j) at col[i]
+            const int64_t last = min(end, j + kd + 1);
+            double t0 = 0.0, t1 = 0.0;
+            int64_t i = c0 + lane;
+            for (; i + 32 < last; i += 64)
+            {
+                t0 += col[i] * y[i];
+                t1 += col[i + 32] * y[i + 32];
+            }
+            if (i < last)
+                t0 += col[i] * y[i];
+            t0 = wsum(t0 + t1);
+            if (lane == 0)
+                s[warp] = y[j] - t0;
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            // M[j][i] = L(j, i): x_i = (s_i - sum_{j > i} L(j, i) x_j) / L(i, i)
+            double v = lane < jb ? s[lane] : 0.0;
+            const double di = inv[lane];
+            v *= di;
+#pragma unroll
+            for (int j = 31; j >= 0; --j)
+            {
+                const double x = __shfl_sync(0xffffffffu, v, j);
+                v -= lane < j ? M[j][lane] * di * x : 0.0;
+            }
+            if (lane < jb)
+                y[j0 + lane] = v;
+        }
+        __syncthreads();
+        fetch(q + 2);
+    }
+    if (lost && threadIdx.x == 0)
+        y[0] = nan(""); // no solution passes for one
 }
 
 // y[d*rank(i)+r] = src[d*i+r]  /  dst[d*i+r] = y[d*rank(i)+r]
@@ -309,7 +637,7 @@ static int32_t direct_setup(Problem &p)
     if ((e = dalloc(p, &p.band_rank, (size_t)n)) != cudaSuccess ||
         (e = dalloc(p, &p.band_y, (size_t)ndof)) != cudaSuccess ||
         (e = dalloc(p, &p.band_fail, 1)) != cudaSuccess ||
-        (e = dalloc(p, &p.band_ab, (size_t)(ldab * ndof))) != cudaSuccess)
+        (e = dalloc(p, &p.band_ab, (size_t)(ldab * ndof) + 1)) != cudaSuccess) // + 1: whole 16-byte copies
     {
         (void)cudaGetLastError(); // a failed allocation is reported here, not by a later launch check
         p.band_ab = nullptr;
@@ -338,21 +666,19 @@ static cudaError_t factor(Problem &p)
     k_band_fill<D><<<div_up(p.n, 128), 128, 0, p.stream>>>(p.n, p.cstart, p.iperm, p.slice_off, p.col_sell, p.K,
                                                           p.band_rank, ldab, p.band_ab);
     p.ctr.kernel_launches++;
-    for (int64_t j0 = 0; j0 < ndof; j0 += kBandNB)
-    {
-        const int64_t jb = std::min<int64_t>(kBandNB, ndof - j0);
-        const int64_t m2 = band::below_end(ndof, kd, j0, jb) - (j0 + jb);
-        k_potrf<<<1, 32, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, p.band_fail);
-        p.ctr.kernel_launches++;
-        if (m2 > 0)
-        {
-            k_trsm<<<(unsigned)div_up(m2, 128), 128, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, m2);
-            const dim3 grid((unsigned)div_up(m2, 128), (unsigned)std::min<int64_t>(m2, 65535));
-            k_syrk<<<grid, 128, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, m2);
-            p.ctr.kernel_launches += 2;
-        }
-    }
-    return cudaGetLastError();
+    if ((e = cudaGetLastError()) != cudaSuccess)
+        return e;
+    if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), p.stream)) != cudaSuccess)
+        return e;
+    double *ab = p.band_ab;
+    int64_t ld = ldab, k = kd, nn = ndof;
+    int *fail = p.band_fail;
+    unsigned *bar = p.barrier;
+    void *args[] = {&ab, &ld, &k, &nn, &fail, &bar};
+    e = cudaLaunchCooperativeKernel((const void *)k_band_factor, dim3(p.num_sms), dim3(kFactorThreads), args,
+                                    kFactorSmem, p.stream);
+    p.ctr.kernel_launches++;
+    return e;
 }
 
 // Forward and backward substitution of p.res into p.x.
@@ -363,30 +689,17 @@ static cudaError_t substitute(Problem &p)
     const int nb = (int)div_up(ndof, 256);
     k_band_perm<<<nb, 256, 0, p.stream>>>(p.n, D, p.band_rank, p.res, p.band_y, 0);
     p.ctr.kernel_launches++;
-    for (int64_t j0 = 0; j0 < ndof; j0 += kBandNB)
+    if (kBandNB * ldab * 8 <= kSolvePanelBytes)
     {
-        const int64_t jb = std::min<int64_t>(kBandNB, ndof - j0);
-        const int64_t m2 = band::below_end(ndof, kd, j0, jb) - (j0 + jb);
-        k_fwd_block<<<1, 1, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, p.band_y);
-        p.ctr.kernel_launches++;
-        if (m2 > 0)
-        {
-            k_fwd_update<<<(unsigned)div_up(m2, 128), 128, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, m2, p.band_y);
-            p.ctr.kernel_launches++;
-        }
+        const cudaError_t e = cudaFuncSetAttribute(k_band_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   2 * kSolvePanelBytes);
+        if (e != cudaSuccess)
+            return e;
+        k_band_solve<true><<<1, kSolveThreads, 2 * kSolvePanelBytes, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y);
     }
-    const int64_t last = ((ndof - 1) / kBandNB) * kBandNB;
-    for (int64_t j0 = last; j0 >= 0; j0 -= kBandNB)
-    {
-        const int64_t jb = std::min<int64_t>(kBandNB, ndof - j0);
-        if (j0 + jb < ndof)
-        {
-            k_bwd_update<<<1, kBandNB, 0, p.stream>>>(p.band_ab, ldab, kd, ndof, j0, jb, p.band_y);
-            p.ctr.kernel_launches++;
-        }
-        k_bwd_block<<<1, 1, 0, p.stream>>>(p.band_ab, ldab, kd, j0, jb, p.band_y);
-        p.ctr.kernel_launches++;
-    }
+    else
+        k_band_solve<false><<<1, kSolveThreads, 0, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y);
+    p.ctr.kernel_launches++;
     k_band_perm<<<nb, 256, 0, p.stream>>>(p.n, D, p.band_rank, p.band_y, p.x, 1);
     p.ctr.kernel_launches++;
     return cudaGetLastError();
@@ -411,6 +724,12 @@ int32_t solve_direct(Problem &p)
         {
             set_last_error(std::string("direct solver: ") + cudaGetErrorString(e));
             return LPMGPU_ERR_CUDA;
+        }
+        if (fail < 0)
+        {
+            p.band_factored = -1;
+            set_last_error("direct solver: a device-side barrier wait timed out");
+            return LPMGPU_ERR_TIMEOUT;
         }
         if (fail)
         {
