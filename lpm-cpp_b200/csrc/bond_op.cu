@@ -374,7 +374,7 @@ __device__ bool bond_allreduce(unsigned *bar, unsigned &epoch, int64_t *info, vo
 // 64 registers hold no more without spills (two bonds spilled: 70 us per iteration on the cube below;
 // 512 threads with two bonds: 25.1 us).  Measured per iteration against k_cg on the assembled matrix:
 // 51x50x50 simple cubic FP64 98.2 -> 23.1 us (its matrix streams 584 MB at 93% of HBM; its bonds are
-// 64 MB), 40x40x40-cell BCC FP32 47.3 -> 15.0 us, 125x144 hexagonal FP64 10.2 -> 9.7 us.
+// 64 MB), 125x144 hexagonal FP64 10.2 -> 9.7 us.
 constexpr int kBondThreads = 1024;
 
 template <typename TV, int D, bool GEN>
@@ -1306,12 +1306,15 @@ cudaError_t setup_bond_op(Problem &p)
     p.bo_nc = (ncmax > 0 && G <= 31 && cluster_smem_of(p, G, G * (32 >> lc)) <= kClusterSmem) ? ncmax : 0;
     while (p.bo_nc > p.bo_ng)
         p.bo_nc /= 2;
+    const bool grid_used = p.desc.precision != LPMGPU_MIXED || p.dim == 2; // solve_dim's rule
     if (p.bo_nc == 0)
         shape(lg);
+    if (p.bo_nc == 0 && !grid_used)
+        return cudaSuccess;
     // one allocation for all arrays, each on a 256-byte boundary, sized for either shape
     const size_t n = (size_t)p.n;
     const int rs = 4 * p.dim + p.dim * (p.dim + 1) / 2;
-    const bool mixed = p.desc.precision == LPMGPU_MIXED;
+    const bool mixed = p.desc.precision == LPMGPU_MIXED && p.dim == 2;
     size_t ent = (size_t)p.bo_ng * p.bo_width * 32, ngr = (size_t)p.bo_ng;
     if (p.bo_nc > 0)
     {
@@ -1368,7 +1371,7 @@ cudaError_t setup_bond_op(Problem &p)
         if ((e = fill()) != cudaSuccess)
             return e;
     }
-    p.bo_ok = hbad == 0;
+    p.bo_ok = hbad == 0 && (p.bo_nc > 0 || grid_used);
     return cudaSuccess;
 }
 
@@ -1551,7 +1554,9 @@ cudaError_t enqueue_bond_grid(Problem &p, const TV *b, TV *x, TV *r, TV *pa, TV 
     s.pb = pb;
     if (p.dim == 2)
         return p.bo_gen ? launch_grid<TV, 2, true>(p, s) : launch_grid<TV, 2, false>(p, s);
-    return p.bo_gen ? launch_grid<TV, 3, true>(p, s) : launch_grid<TV, 3, false>(p, s);
+    if constexpr (sizeof(TV) == 8)
+        return p.bo_gen ? launch_grid<TV, 3, true>(p, s) : launch_grid<TV, 3, false>(p, s);
+    return cudaErrorInvalidValue; // FP32 in 3D runs on the assembled matrix (solve_dim)
 }
 template cudaError_t enqueue_bond_grid<double>(Problem &, const double *, double *, double *, double *, double *, double,
                                                double, double, int64_t);
@@ -1571,7 +1576,9 @@ cudaError_t bond_default_grid(const Problem &p, int *grid)
     }
     if (p.dim == 2)
         return p.bo_gen ? bond_grid<TV, 2, true>(p, grid) : bond_grid<TV, 2, false>(p, grid);
-    return p.bo_gen ? bond_grid<TV, 3, true>(p, grid) : bond_grid<TV, 3, false>(p, grid);
+    if constexpr (sizeof(TV) == 8)
+        return p.bo_gen ? bond_grid<TV, 3, true>(p, grid) : bond_grid<TV, 3, false>(p, grid);
+    return cudaErrorInvalidValue;
 }
 template cudaError_t bond_default_grid<double>(const Problem &, int *);
 template cudaError_t bond_default_grid<float>(const Problem &, int *);
