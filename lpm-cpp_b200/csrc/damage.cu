@@ -102,13 +102,13 @@ static cudaError_t build_nonlocal_grid(Problem &p, double rc)
                 cudaFreeAsync(q, p.stream);
     };
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&d_cxyz, sizeof(int) * cxyz.size(), p.stream);
+        e = pool_alloc(&d_cxyz, sizeof(int) * cxyz.size(), p.stream);
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&d_cs, sizeof(int) * cell_start.size(), p.stream);
+        e = pool_alloc(&d_cs, sizeof(int) * cell_start.size(), p.stream);
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&d_ci, sizeof(int) * cell_ids.size(), p.stream);
+        e = pool_alloc(&d_ci, sizeof(int) * cell_ids.size(), p.stream);
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&cnt, sizeof(int) * ((size_t)n + 1), p.stream);
+        e = pool_alloc(&cnt, sizeof(int) * ((size_t)n + 1), p.stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_cxyz, cxyz.data(), sizeof(int) * cxyz.size(), cudaMemcpyHostToDevice, p.stream);
     if (e == cudaSuccess)
@@ -139,7 +139,7 @@ static cudaError_t build_nonlocal_grid(Problem &p, double rc)
     if (e == cudaSuccess)
         e = dalloc(p, &p.ddot_nonlocal, (size_t)n);
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&unsorted, sizeof(int) * ((size_t)total + 1), p.stream);
+        e = pool_alloc(&unsorted, sizeof(int) * ((size_t)total + 1), p.stream);
     if (e == cudaSuccess)
     {
         k_nonlocal_grid<1><<<div_up(n, 128), 128, 0, p.stream>>>(n, p.xyz, rc, d_cxyz, dims[0], dims[1], dims[2], d_cs,
@@ -164,7 +164,7 @@ cudaError_t build_nonlocal(Problem &p, double cutoff_ratio)
     if (e != cudaSuccess)
         return e;
     int *cnt = nullptr;
-    if ((e = cudaMallocAsync(&cnt, sizeof(int) * ((size_t)n + 1), p.stream)) != cudaSuccess)
+    if ((e = pool_alloc(&cnt, sizeof(int) * ((size_t)n + 1), p.stream)) != cudaSuccess)
         return e;
     if ((e = cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)n + 1), p.stream)) != cudaSuccess)
         return e;

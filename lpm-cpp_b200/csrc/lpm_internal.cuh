@@ -252,12 +252,26 @@ void set_last_error(const std::string &s);
 // flushes and frees the handle's dump writer (waits for the steps it still writes)
 void release_dump_writer(Problem &p);
 
+// the library's memory pool (memory.cu): device memory ordered on a stream, given back by cudaFreeAsync,
+// and blocks of pinned host memory for a problem's scalar record and status words
+cudaError_t pool_alloc_bytes(void **ptr, size_t bytes, cudaStream_t st);
+template <typename T>
+cudaError_t pool_alloc(T **ptr, size_t bytes, cudaStream_t st)
+{
+    void *v = nullptr;
+    const cudaError_t e = pool_alloc_bytes(&v, bytes, st);
+    *ptr = static_cast<T *>(v);
+    return e;
+}
+cudaError_t pinned_take(void **ptr);
+void pinned_give(void *ptr);
+
 template <typename T>
 cudaError_t dalloc(Problem &p, T **ptr, size_t count)
 {
     void *v = nullptr;
     size_t bytes = sizeof(T) * (count ? count : 1);
-    cudaError_t e = cudaMalloc(&v, bytes);
+    cudaError_t e = pool_alloc_bytes(&v, bytes, p.stream);
     if (e != cudaSuccess)
         return e;
     p.allocs.push_back(v);

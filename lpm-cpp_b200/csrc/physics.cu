@@ -583,7 +583,7 @@ cudaError_t launch_apply_bc(Problem &p, const lpmgpu_load_step &s)
     if (total == 0)
         return cudaSuccess;
     int *dids = nullptr;
-    cudaError_t e = cudaMallocAsync(&dids, sizeof(int) * total, p.stream);
+    cudaError_t e = pool_alloc(&dids, sizeof(int) * total, p.stream);
     if (e != cudaSuccess)
         return e;
     std::vector<int> h(total);

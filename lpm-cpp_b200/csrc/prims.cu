@@ -135,7 +135,7 @@ cudaError_t scan_impl(cudaStream_t st, const T *in, T *out, int64_t count)
         return cudaSuccess;
     const int64_t tiles = (count + kScanTile - 1) / kScanTile;
     T *sums = nullptr, *offs = nullptr;
-    cudaError_t e = cudaMallocAsync(&sums, sizeof(T) * 2 * tiles, st);
+    cudaError_t e = pool_alloc(&sums, sizeof(T) * 2 * tiles, st);
     if (e != cudaSuccess)
         return e;
     offs = sums + tiles;
@@ -329,7 +329,7 @@ cudaError_t prim_sort_pairs(cudaStream_t st, const int *key, const int *val, int
         return cudaSuccess;
     const int64_t N = sort_size(n);
     unsigned long long *k64 = nullptr;
-    cudaError_t e = cudaMallocAsync(&k64, sizeof(unsigned long long) * N, st);
+    cudaError_t e = pool_alloc(&k64, sizeof(unsigned long long) * N, st);
     if (e != cudaSuccess)
         return e;
     k_pack_pairs<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(key, n, N, k64);
@@ -348,7 +348,7 @@ cudaError_t prim_segmented_sort(cudaStream_t st, const int *in, int *out, int64_
         return cudaSuccess;
     const int64_t N = sort_size(total);
     unsigned long long *k64 = nullptr;
-    cudaError_t e = cudaMallocAsync(&k64, sizeof(unsigned long long) * N, st);
+    cudaError_t e = pool_alloc(&k64, sizeof(unsigned long long) * N, st);
     if (e != cudaSuccess)
         return e;
     k_pack_segments<<<1024, 256, 0, st>>>(in, nseg, off, total, N, k64);

@@ -664,12 +664,12 @@ static void free_problem(Problem &p)
                 slots[k] = nullptr;
             }
     for (void *v : p.allocs)
-        cudaFree(v);
+        cudaFreeAsync(v, p.stream);
     p.allocs.clear();
+    if (p.stream)
+        cudaStreamSynchronize(p.stream);
     if (p.scal_host)
-        cudaFreeHost(p.scal_host);
-    if (p.cg_info_host)
-        cudaFreeHost(p.cg_info_host);
+        pinned_give(p.scal_host);
     for (auto &e : p.ev)
         if (e)
             cudaEventDestroy(e);
@@ -754,8 +754,11 @@ int32_t lpmgpu_create(const lpmgpu_desc *d, lpmgpu_solver **out)
     else
         kntv(p.cell, d->plane_stress, d->E, d->mu, p.kntv);
     const size_t n = p.n;
-    CKF(cudaMallocHost(&p.scal_host, sizeof(Scalars)));
-    CKF(cudaMallocHost(&p.cg_info_host, 8 * sizeof(int64_t)));
+    void *pinned = nullptr;
+    CKF(pinned_take(&pinned));
+    p.scal_host = static_cast<Scalars *>(pinned);
+    p.cg_info_host = reinterpret_cast<int64_t *>(static_cast<char *>(pinned) + 128);
+    std::memset(pinned, 0, 256);
     CKF(dalloc(p, &p.scal, 1));
     CKF(dalloc(p, &p.partials, 2 * std::max<size_t>((size_t)kMaxGridBlocks, n / 64 + 1) + 16));
     CKF(dalloc(p, &p.barrier, 4));

@@ -554,9 +554,9 @@ static cudaError_t spread_slices(Problem &p, int64_t *width)
     if (!moved)
         return cudaSuccess;
     int *d_order = nullptr, *perm2 = nullptr;
-    if ((e = cudaMallocAsync(&d_order, sizeof(int) * nmove, p.stream)) != cudaSuccess)
+    if ((e = pool_alloc(&d_order, sizeof(int) * nmove, p.stream)) != cudaSuccess)
         return e;
-    if ((e = cudaMallocAsync(&perm2, sizeof(int) * (size_t)nmove * kSlice, p.stream)) != cudaSuccess)
+    if ((e = pool_alloc(&perm2, sizeof(int) * (size_t)nmove * kSlice, p.stream)) != cudaSuccess)
         return e;
     e = cudaMemcpyAsync(d_order, order.data(), sizeof(int) * nmove, cudaMemcpyHostToDevice, p.stream);
     if (e == cudaSuccess)
@@ -585,7 +585,7 @@ static cudaError_t exclusive_scan(Problem &p, const T *in, T *out, int count)
 static cudaError_t reduce_max(Problem &p, const int *in, int count, int *host_out)
 {
     int *dmax = nullptr;
-    cudaError_t e = cudaMallocAsync(&dmax, sizeof(int), p.stream);
+    cudaError_t e = pool_alloc(&dmax, sizeof(int), p.stream);
     if (e != cudaSuccess)
         return e;
     e = prim_max(p.stream, in, count, dmax);
@@ -647,12 +647,12 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
     }
 
     int *key = nullptr, *ids = nullptr, *skey = nullptr, *sid = nullptr, *cbeg = nullptr, *cend = nullptr;
-    LPM_TRY(cudaMallocAsync(&key, sizeof(int) * n, p.stream));
-    LPM_TRY(cudaMallocAsync(&ids, sizeof(int) * n, p.stream));
-    LPM_TRY(cudaMallocAsync(&skey, sizeof(int) * n, p.stream));
-    LPM_TRY(cudaMallocAsync(&sid, sizeof(int) * n, p.stream));
-    LPM_TRY(cudaMallocAsync(&cbeg, sizeof(int) * ncell, p.stream));
-    LPM_TRY(cudaMallocAsync(&cend, sizeof(int) * ncell, p.stream));
+    LPM_TRY(pool_alloc(&key, sizeof(int) * n, p.stream));
+    LPM_TRY(pool_alloc(&ids, sizeof(int) * n, p.stream));
+    LPM_TRY(pool_alloc(&skey, sizeof(int) * n, p.stream));
+    LPM_TRY(pool_alloc(&sid, sizeof(int) * n, p.stream));
+    LPM_TRY(pool_alloc(&cbeg, sizeof(int) * ncell, p.stream));
+    LPM_TRY(pool_alloc(&cend, sizeof(int) * ncell, p.stream));
     LPM_TRY(cudaMemsetAsync(cbeg, 0, sizeof(int) * ncell, p.stream));
     LPM_TRY(cudaMemsetAsync(cend, 0, sizeof(int) * ncell, p.stream));
     const int T = 256;
@@ -664,8 +664,8 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
 
     int *pad_id = nullptr;
     double *pad_d = nullptr;
-    LPM_TRY(cudaMallocAsync(&pad_id, sizeof(int) * (size_t)n * kMaxBonds, p.stream));
-    LPM_TRY(cudaMallocAsync(&pad_d, sizeof(double) * (size_t)n * kMaxBonds, p.stream));
+    LPM_TRY(pool_alloc(&pad_id, sizeof(int) * (size_t)n * kMaxBonds, p.stream));
+    LPM_TRY(pool_alloc(&pad_d, sizeof(double) * (size_t)n * kMaxBonds, p.stream));
     LPM_TRY(dalloc(p, &p.nb, n));
     LPM_TRY(dalloc(p, &p.nb0, n));
     LPM_TRY(dalloc(p, &p.bstart, (size_t)n + 1));
@@ -707,7 +707,7 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
     LPM_TRY(cudaGetLastError());
     // bstart = exclusive scan of nb (n+1 entries: the appended zero yields the total)
     int *nbx = nullptr;
-    LPM_TRY(cudaMallocAsync(&nbx, sizeof(int) * ((size_t)n + 1), p.stream));
+    LPM_TRY(pool_alloc(&nbx, sizeof(int) * ((size_t)n + 1), p.stream));
     LPM_TRY(cudaMemsetAsync(nbx, 0, sizeof(int) * ((size_t)n + 1), p.stream));
     LPM_TRY(cudaMemcpyAsync(nbx, p.nb, sizeof(int) * n, cudaMemcpyDeviceToDevice, p.stream));
     LPM_TRY(exclusive_scan(p, nbx, p.bstart, n + 1));
@@ -764,8 +764,8 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
 
     // connections
     int *pad_c = nullptr, *ncx = nullptr;
-    LPM_TRY(cudaMallocAsync(&pad_c, sizeof(int) * (size_t)n * kMaxConns, p.stream));
-    LPM_TRY(cudaMallocAsync(&ncx, sizeof(int) * ((size_t)n + 1), p.stream));
+    LPM_TRY(pool_alloc(&pad_c, sizeof(int) * (size_t)n * kMaxConns, p.stream));
+    LPM_TRY(pool_alloc(&ncx, sizeof(int) * ((size_t)n + 1), p.stream));
     LPM_TRY(cudaMemsetAsync(ncx, 0, sizeof(int) * ((size_t)n + 1), p.stream));
     LPM_TRY(dalloc(p, &p.nlq, n));
     LPM_TRY(dalloc(p, &p.cstart, (size_t)n + 1));
@@ -801,16 +801,16 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
     // each slice width spread over the slice order
     {
         int *key = nullptr, *ids = nullptr, *skey = nullptr;
-        LPM_TRY(cudaMallocAsync(&key, sizeof(int) * n, p.stream));
-        LPM_TRY(cudaMallocAsync(&ids, sizeof(int) * n, p.stream));
-        LPM_TRY(cudaMallocAsync(&skey, sizeof(int) * n, p.stream));
+        LPM_TRY(pool_alloc(&key, sizeof(int) * n, p.stream));
+        LPM_TRY(pool_alloc(&ids, sizeof(int) * n, p.stream));
+        LPM_TRY(pool_alloc(&skey, sizeof(int) * n, p.stream));
         LPM_TRY(dalloc(p, &p.perm, n));
         LPM_TRY(dalloc(p, &p.iperm, n));
         k_sell_keys<<<div_up(n, T), T, 0, p.stream>>>(n, p.cstart, key, ids);
         LPM_TRY(prim_sort_pairs(p.stream, key, ids, skey, p.perm, n));
         p.nslices = div_up(n, kSlice);
         int64_t *width = nullptr;
-        LPM_TRY(cudaMallocAsync(&width, sizeof(int64_t) * (p.nslices + 1), p.stream));
+        LPM_TRY(pool_alloc(&width, sizeof(int64_t) * (p.nslices + 1), p.stream));
         LPM_TRY(dalloc(p, &p.slice_off, (size_t)p.nslices + 1));
         k_sell_width<<<div_up(p.nslices + 1, T), T, 0, p.stream>>>(n, p.nslices, p.perm, p.cstart, nullptr, width);
         LPM_TRY(cudaGetLastError());
@@ -832,7 +832,7 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
 
     // reference K_pointer
     int64_t *kv = nullptr;
-    LPM_TRY(cudaMallocAsync(&kv, sizeof(int64_t) * ((size_t)n + 1), p.stream));
+    LPM_TRY(pool_alloc(&kv, sizeof(int64_t) * ((size_t)n + 1), p.stream));
     LPM_TRY(dalloc(p, &p.kp_ref, (size_t)n + 1));
     k_kp_counts<<<div_up(n + 1, T), T, 0, p.stream>>>(n, p.dim, p.nlq, kv);
     LPM_TRY(exclusive_scan(p, kv, p.kp_ref, n + 1));
