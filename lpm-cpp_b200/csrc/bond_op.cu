@@ -329,44 +329,6 @@ __device__ __forceinline__ void general_close(const RowTerms<TV, D> &rt, const T
                          TV(0.25) * (rt.v[2 * D + k] * G0 + rt.v[3 * D + k] * G1));
 }
 
-// Grid barrier + all-reduce of per-block partials, as grid_allreduce of cg.cu: the word only counts
-// arrivals, every block sums all partials in one order.  false: a wait passed its limit.
-__device__ bool bond_allreduce(unsigned *bar, unsigned &epoch, int64_t *info, volatile int *s_fail,
-                               const double *part, int slot, double *sh, double *out, unsigned long long wait_ns)
-{
-    __shared__ double s_tot;
-    if (threadIdx.x == 0)
-    {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const unsigned target = (epoch + 1u) * gridDim.x;
-        const unsigned long long t0 = gtimer();
-        while ((int)(ld_acquire(bar) - target) < 0)
-            if (gtimer() - t0 > wait_ns)
-            {
-                atomicOr(reinterpret_cast<unsigned long long *>(info + 1), 2ull);
-                *s_fail = 1;
-                break;
-            }
-    }
-    epoch++;
-    __syncthreads();
-    if (*s_fail)
-        return false;
-    if (threadIdx.x < 32)
-    {
-        double v = 0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
-            v += __ldcg(part + 2 * b + slot);
-        v = wsum(v);
-        if (threadIdx.x == 0)
-            s_tot = v;
-    }
-    __syncthreads();
-    *out = s_tot;
-    return true;
-}
-
 // The CG on the whole grid, one block per SM, each owning a contiguous share of the groups.  Bound by
 // the bond stream (28 bytes per bond and pass in FP64 3D, twice per iteration, from L2 while it fits
 // there) and its gathers, plus two grid barriers of about 2.5 us.  pq is known after pass 1, so x and r
@@ -417,9 +379,8 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
             st_vec<TV, D>(s.pa, n, i, zero, pl);
         }
     }
-    block_partial(loc, s.part, 0, sh);
     double rr;
-    if (!bond_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, s.wait_ns))
+    if (!grid_sum(loc, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, s.wait_ns))
         return;
     const double stop = (s.abs_stop >= 0) ? s.abs_stop : s.rtol * rr + s.atol;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -526,9 +487,8 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                     st_keep2(s.th + 2 * (int64_t)i, make_float2(a0, a1), pl);
             }
         }
-        block_partial(lpq, s.part, 1, sh);
         double pq;
-        if (!bond_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
+        if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
             return;
         if (pq == 0.0)
         {
@@ -658,9 +618,8 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                 st_vec<TV, D>(s.r, n, i, rv, pl);
             }
         }
-        block_partial(lrr, s.part, 0, sh);
         double rn;
-        if (!bond_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, s.wait_ns))
+        if (!grid_sum(lrr, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, s.wait_ns))
             return;
         const bool done = rn <= stop;
         if (done || it >= s.maxit)

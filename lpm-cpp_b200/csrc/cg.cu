@@ -55,60 +55,6 @@ struct CGState
 };
 
 
-// Grid barrier + all-reduce of the per-block partials part[2*b + slot], with nothing serial on
-// the way out: the barrier word only counts arrivals (it starts at zero and is never reset, so
-// barrier number e is passed once it reaches (e + 1) * gridDim.x), and after it every block
-// sums all partials itself, in one fixed order (thread t takes b = t, t + blockDim, ..., warp
-// butterflies, then thread 0 over the warp sums in order), so every block holds the same
-// bit-identical total.  The two slots alternate between consecutive reductions, which keeps a
-// block that runs one phase ahead from overwriting partials another block is still reading.
-// Returns false when the wait timed out (the status word gets bit 2).
-__device__ bool grid_allreduce(unsigned *bar, unsigned &epoch, int64_t *info, volatile int *s_fail,
-                               const double *part, int slot, double *sh, double *out,
-                               unsigned long long wait_ns)
-{
-    __shared__ double s_tot;
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const unsigned target = (epoch + 1u) * gridDim.x;
-        const unsigned long long t0 = gtimer();
-        while ((int)(ld_acquire(bar) - target) < 0)
-        {
-            if (gtimer() - t0 > wait_ns)
-            {
-                atomicOr(reinterpret_cast<unsigned long long *>(info + 1), 2ull);
-                *s_fail = 1;
-                break;
-            }
-        }
-    }
-    epoch++;
-    __syncthreads();
-    if (*s_fail)
-        return false;
-    double v = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-        v += __ldcg(part + 2 * b + slot);
-    v = wsum(v);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0)
-        sh[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        double t = 0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q)
-            t += sh[q];
-        s_tot = t;
-    }
-    __syncthreads();
-    *out = s_tot;
-    return true;
-}
-
 template <typename TK, typename TV, int D>
 __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, const TK *__restrict__ K, const TV *__restrict__ b,
                                                    TV *__restrict__ x, TV *__restrict__ r, TV *__restrict__ pa,
@@ -138,9 +84,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
         st_keep(pa + k, TV(0), pl);
         loc += (double)v * (double)v;
     }
-    block_partial(loc, s.part, 0, sh);
     double rr;
-    if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, s.wait_ns))
+    if (!grid_sum(loc, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, s.wait_ns))
         return;
     const double stop = (s.abs_stop >= 0) ? s.abs_stop : s.rtol * rr + s.atol;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -157,9 +102,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
     {
         const double lpq = spmv_block<TK, TV, D>(s0, s1, s.n, s.rowptr, s.perm, s.slice_off, s.col_sell, K, r,
                                                    pold, pnew, q, beta, pf, pl, red);
-        block_partial(lpq, s.part, 1, sh);
         double pq;
-        if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
+        if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
             return;
         if (pq == 0.0)
         {
@@ -181,9 +125,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
             st_keep(r + k, rv, pl);
             lrr += (double)rv * (double)rv;
         }
-        block_partial(lrr, s.part, 0, sh);
         double rn;
-        if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, s.wait_ns))
+        if (!grid_sum(lrr, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, s.wait_ns))
             return;
         const bool done = rn <= stop;
         const bool capped = it >= s.maxit;
@@ -828,9 +771,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
         st_keep(pa + k, 0.0, pl);
         loc += v * v;
     }
-    block_partial(loc, s.part, 0, sh);
     double rr;
-    if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, kBarrierTimeoutNs))
+    if (!grid_sum(loc, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, kBarrierTimeoutNs))
         return;
     const double stop = s.rtol * rr + s.atol;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -854,9 +796,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
                 lpq += pn * qv;
             }
         }
-        block_partial(lpq, s.part, 1, sh);
         double pq;
-        if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, kBarrierTimeoutNs))
+        if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, kBarrierTimeoutNs))
             return;
         if (pq == 0.0)
         {
@@ -876,9 +817,8 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
             st_keep(r + k, rv, pl);
             lrr += rv * rv;
         }
-        block_partial(lrr, s.part, 0, sh);
         double rn;
-        if (!grid_allreduce(s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, kBarrierTimeoutNs))
+        if (!grid_sum(lrr, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, kBarrierTimeoutNs))
             return;
         if (rn <= stop || it >= s.maxit)
         {
