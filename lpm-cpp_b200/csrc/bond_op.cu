@@ -8,7 +8,7 @@
 #include <type_traits>
 
 #include "bond_op.cuh"
-#include "cg_device.cuh"
+#include "cluster.cuh"
 
 namespace lpm
 {
@@ -652,36 +652,11 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
 // warp owns no rows: it exchanges the sums, p . K p while the others run pass 2 (which needs theta,
 // but alpha only at its end).
 //
-// Bound by latency below about 200 rows per CTA (an exchange takes 366 cycles whatever the cluster's
-// size; a release/acquire cluster barrier with remote stores took 1,070 at 16 CTAs) and by shared-memory
-// bandwidth above (20 wavefronts per 32 bonds in 2D and iteration).  Measured per iteration against
+// Bound by latency below about 200 rows per CTA and by shared-memory bandwidth above (20 wavefronts per 32 bonds in 2D and iteration).  Measured per iteration against
 // k_cg on the assembled matrix: hexagonal plates of 725, 2,900 and 11,500 particles 7.9 -> 2.9,
 // 8.3 -> 3.3 and 9.9 -> 5.6 us; simple-cubic cubes of 1,728 and 4,096 particles 9.8 -> 4.1 and
 // 10.6 -> 5.4 us.  Gathering the neighbours from other CTAs' shared memory instead took 4.0, 5.2 and
 // 7.8 us on the plates.
-__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned mapa(unsigned a, unsigned rank)
-{
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void push(unsigned dst, unsigned bar, double v)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(dst), "d"(v), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void push2(unsigned dst, unsigned bar, double a, double b)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(dst), "d"(a),
-                 "d"(b), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 struct ClusterShared
 {
     double part[2][16]; // partial sums of the CTAs: [0] r.r, [1] p.Kp
@@ -699,43 +674,6 @@ constexpr int kHeldBytes = 8 * D + (GEN ? 32 : 16);
 template <int D, bool GEN>
 constexpr int kSlotBytes = 32 * (4 + 8 * D + (GEN ? 16 : 0));
 constexpr size_t kClusterFixed = (sizeof(ClusterShared) + 127) / 128 * 128;
-constexpr size_t kClusterSmem = 232448; // shared memory of one CTA on sm_100
-
-// Waits until the phase `parity` of an mbarrier of this CTA is complete; false once the limit passed.
-__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, unsigned long long wait_ns)
-{
-    unsigned long long t0 = 0;
-    while (true)
-    {
-        unsigned done;
-        if (wait_ns >= 100000ull)
-            asm volatile("{\n.reg .pred p;\n"
-                         "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                         "selp.u32 %0, 1, 0, p;\n}"
-                         : "=r"(done)
-                         : "r"(bar), "r"(parity)
-                         : "memory");
-        else // a try may sleep past a limit this short
-            asm volatile("{\n.reg .pred p;\n"
-                         "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                         "selp.u32 %0, 1, 0, p;\n}"
-                         : "=r"(done)
-                         : "r"(bar), "r"(parity)
-                         : "memory");
-        if (done)
-            return true;
-        const unsigned long long now = gtimer();
-        if (t0 == 0)
-            t0 = now;
-        else if (now - t0 > wait_ns)
-            return false;
-    }
-}
-
-__device__ __forceinline__ void expect_bytes(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 
 // The exchange of one sum by one warp: adds the CTA's `nw` warp sums sh[which][.], sends the total
 // to every CTA, waits for theirs (and `halo` bytes of pushes on the same mbarrier) and leaves the
@@ -800,8 +738,8 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
     {
         cs->fail = 1 << 30;
         for (int k = 0; k < 3; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&cs->mbar[k])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            mbar_init(&cs->mbar[k]);
+        mbar_init_done();
     }
     // the rows each CTA holds: its own and all that its bonds reach
     for (int k = warp; k < (int)nc; k += nw)
@@ -1191,35 +1129,6 @@ static const void *cluster_kernel(const Problem &p)
     return p.bo_gen ? (const void *)k_cg_bond_cluster<3, true> : (const void *)k_cg_bond_cluster<3, false>;
 }
 
-// largest cluster the device runs with a CTA's whole shared memory (16, else 8); 0 when none
-static int max_cluster(const void *kernel)
-{
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    {
-        (void)cudaGetLastError();
-        return 0;
-    }
-    for (int nc = 16; nc >= 8; nc /= 2)
-    {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(nc);
-        cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = kClusterSmem;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = nc;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int k = 0;
-        if (cudaOccupancyMaxActiveClusters(&k, kernel, &cfg) == cudaSuccess && k > 0)
-            return nc;
-        (void)cudaGetLastError();
-    }
-    return 0;
-}
-
 // largest cluster for the problem's kernel, asked once per kernel
 static int cluster_limit(const Problem &p)
 {
@@ -1440,23 +1349,8 @@ cudaError_t enqueue_bond_cluster(Problem &p, const double *b, double *x, double 
     s.r = s.pa = s.pb = nullptr;
     const int nc = cluster_ctas(p);
     int G = div_up(p.bo_ng, nc), slots = G * p.bo_width, held = held_rows(p, nc);
-    const void *k = cluster_kernel(p);
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-        return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nc);
-    cfg.blockDim = dim3(32 * (G + 1));
-    cfg.dynamicSmemBytes = cluster_smem_of(p, G, held);
-    cfg.stream = p.stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = nc;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
     void *args[] = {&s, &G, &slots, &held};
-    if ((e = cudaLaunchKernelExC(&cfg, k, args)) != cudaSuccess)
+    if ((e = launch_cluster(cluster_kernel(p), nc, 32 * (G + 1), cluster_smem_of(p, G, held), args, p.stream)) != cudaSuccess)
         return e;
     p.ctr.kernel_launches++;
     p.ctr.cg_launches++;

@@ -32,6 +32,7 @@
 #include <string>
 
 #include "bond_op.cuh"
+#include "cg_cluster.cuh"
 #include "cg_device.cuh"
 
 namespace lpm
@@ -360,6 +361,14 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
             return e;
         }
     }
+    if constexpr (D == 2)
+        if (p.desc.precision != LPMGPU_MIXED && sell_cluster_fits(p))
+        {
+            cudaError_t e = cudaEventRecord(p.cg_ev[0], p.stream);
+            if (e == cudaSuccess)
+                e = enqueue_sell_cluster(p, p.res, p.x, p.desc.cg_rtol, p.desc.cg_atol, -1.0, maxit);
+            return e != cudaSuccess ? e : finish_cg(p, "assembled fp64 cluster", out, nullptr, nullptr);
+        }
     if (p.desc.precision != LPMGPU_MIXED)
         return run_cg<double, double, D>(p, p.K, p.res, p.x, p.r, p.p0, p.p1, p.q, p.desc.cg_rtol, p.desc.cg_atol,
                                          -1.0, maxit, out, nullptr);
@@ -920,7 +929,21 @@ extern "C" int32_t lpmgpu_cg_bsr_noalloc(int32_t dim, int32_t nrows, const int32
     s.maxit = maxit > 0 ? maxit : s.ndof;
     int64_t status[2] = {0, 0};
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    e = (dim == 2) ? noalloc_launch<2>(scr, grid, s, b, x, st, status) : noalloc_launch<3>(scr, grid, s, b, x, st, status);
+    bool solved = false;
+    if (bsr_cluster_may_fit(dim, nrows))
+    {
+        int64_t *info = reinterpret_cast<int64_t *>(scr + 4 * kNoAllocMaxDof + 2 * kNoAllocMaxBlocks);
+        e = cudaMemsetAsync(info, 0, 4 * sizeof(int64_t), st);
+        if (e == cudaSuccess)
+            e = enqueue_bsr_cluster(dim, nrows, rowptr, colidx, values, b, x, rtol, atol, s.maxit, info, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(status, info, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(st);
+        solved = e != cudaSuccess || !(status[1] & kCgDeclined);
+    }
+    if (!solved)
+        e = (dim == 2) ? noalloc_launch<2>(scr, grid, s, b, x, st, status) : noalloc_launch<3>(scr, grid, s, b, x, st, status);
     if (e != cudaSuccess)
     {
         set_last_error(std::string("lpmgpu_cg_bsr_noalloc: ") + cudaGetErrorString(e));
