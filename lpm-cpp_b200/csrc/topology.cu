@@ -452,12 +452,23 @@ __global__ void k_kp_counts(int n, int dim, const int *__restrict__ nlq, int64_t
 }
 
 // ---- sliced-ELL row order and column slots
-__global__ void k_sell_keys(int n, const int *__restrict__ cstart, int *__restrict__ key, int *__restrict__ ids)
+// Rows of a 3D lattice are sorted by descending connection count within windows of this many consecutive
+// rows, not over the whole problem: sorted globally, the slices of a face's rows (lanes a lattice row
+// apart, so every gather of theirs takes 32 sectors) all fall to the last blocks, and the others wait for
+// them at each grid sum.  FP32 CG, us per iteration, whole problem -> windows: FCC 131,072 rows 85.4 ->
+// 59.7 (its power-of-two strides also share cache sets), FCC 129,600 63.0 -> 59.1, BCC 182,250 80.1 ->
+// 75.1, BCC 410,286 126.6 -> 120.6, SC 127,500 58.4 -> 58.8.  32 to 2,048 rows measure alike, 4,096 gives
+// FCC 64.4.  FP64: FCC 131,072 117 -> 101, BCC 182,250 128 -> 112, SC 127,500 98.9 -> 96.3.  A slice is as wide as its longest row; idle lanes of a narrow row load nothing.  2D keeps the
+// whole-problem sort with the slices of each width spread (spread_slices).
+constexpr int kSortWindow = 1024; // a multiple of kSlice
+
+__global__ void k_sell_keys(int n, int window, const int *__restrict__ cstart, int *__restrict__ key,
+                            int *__restrict__ ids)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    key[i] = kMaxConns - (cstart[i + 1] - cstart[i]);
+    key[i] = (i / window) * (kMaxConns + 1) + kMaxConns - (cstart[i + 1] - cstart[i]);
     ids[i] = i;
 }
 
@@ -797,8 +808,8 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
     cudaFreeAsync(pad_c, p.stream);
     cudaFreeAsync(ncx, p.stream);
 
-    // sliced-ELL layout: rows by descending connection count (stable sort), slices of 32; in 2D
-    // each slice width spread over the slice order
+    // sliced-ELL layout: rows by descending connection count (stable sort; in 3D within windows),
+    // slices of 32; in 2D each slice width spread over the slice order
     {
         int *key = nullptr, *ids = nullptr, *skey = nullptr;
         LPM_TRY(pool_alloc(&key, sizeof(int) * n, p.stream));
@@ -806,7 +817,8 @@ cudaError_t build_topology(Problem &p, const double *xyz_host, int *err_code)
         LPM_TRY(pool_alloc(&skey, sizeof(int) * n, p.stream));
         LPM_TRY(dalloc(p, &p.perm, n));
         LPM_TRY(dalloc(p, &p.iperm, n));
-        k_sell_keys<<<div_up(n, T), T, 0, p.stream>>>(n, p.cstart, key, ids);
+        const int window = p.dim == 3 ? std::min(n, kSortWindow) : n;
+        k_sell_keys<<<div_up(n, T), T, 0, p.stream>>>(n, window, p.cstart, key, ids);
         LPM_TRY(prim_sort_pairs(p.stream, key, ids, skey, p.perm, n));
         p.nslices = div_up(n, kSlice);
         int64_t *width = nullptr;
