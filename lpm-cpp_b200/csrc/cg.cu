@@ -32,6 +32,7 @@
 #include <string>
 
 #include "bond_op.cuh"
+#include "bulk_copy.cuh"
 #include "cg_cluster.cuh"
 #include "cg_device.cuh"
 
@@ -148,6 +149,220 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
         pold = pnew;
         pnew = t;
     }
+}
+
+// The FP32 CG of a 3D problem large enough that a warp owns whole slices in every block (k_cg's rule on
+// column splits): the same sums in the same order, so the same bits, with the matrix streamed to shared
+// memory by bulk copies.  k_cg holds a step's nine matrix loads and six gathers per lane in registers,
+// which bounds it by the latency of the gathers at two steps in flight (DRAM at 55 % of its peak).  Here a
+// warp's matrix comes in chunks of kStreamCols block columns (1,152 bytes each), refilled as soon as a
+// chunk is used, over the ends of slices and over the grid sums, and the registers hold the gathers of a
+// whole chunk.  Chunks of 1 / 2 / 3 / 4 / 5 columns: 131 / 115.5 / 112.2 / 114.2 / 120 us per iteration
+// at 410,286 BCC rows (672 MB of matrix; more chunks per warp measure the same: a copy is never waited
+// for long).  k_cg -> this: BCC 410,286 rows 123 -> 112 us, BCC 182,250 75.0 -> 60.3, FCC 131,072 60.1 ->
+// 55.6, SC 127,500 59.2 -> 52.5.  A direction formed by its own pass before the product, which halves
+// the gathers for a third grid sum: 111.6, 61.3, 56.7, 53.1.
+constexpr int kStreamCols = 3;
+constexpr size_t kStreamSmem = (size_t)32 * kStreamCols * 9 * kSlice * sizeof(float);
+
+__global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
+    k_cg_stream(CGState s, const float *__restrict__ K, const float *__restrict__ b, float *__restrict__ x,
+                float *__restrict__ r, float *__restrict__ pa, float *__restrict__ pb, float *__restrict__ q)
+{
+    constexpr int D = 3, E = 9, C = kStreamCols;
+    extern __shared__ __align__(128) float ring[];
+    __shared__ uint64_t full[32];
+    __shared__ double sh[32];
+    __shared__ int s_fail;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s0 = (int)((int64_t)blockIdx.x * s.nslices / gridDim.x);
+    const int s1 = (int)((int64_t)(blockIdx.x + 1) * s.nslices / gridDim.x);
+    const int64_t T = (int64_t)gridDim.x * blockDim.x;
+    const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t pf = l2_evict_first(), pl = l2_evict_last();
+    const bool has = s0 + warp < s1;
+    float *mine = ring + (size_t)warp * C * E * kSlice;
+    uint64_t *bar = full + warp;
+    if (threadIdx.x == 0)
+        s_fail = 0;
+    if (lane == 0)
+    {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    // the next chunk to fetch (lane 0): columns [pk, pk + C) of slice psl, which has pw columns at pkp
+    int psl = s0 + warp, pk = 0, pw = 0;
+    const float *pkp = K;
+    auto slice_of = [&]() {
+        const int64_t off = s.slice_off[psl];
+        pw = (int)(s.slice_off[psl + 1] - off);
+        pkp = K + off * E * kSlice;
+        pk = 0;
+    };
+    auto issue = [&]() {
+        const uint32_t bytes = (uint32_t)(min(C, pw - pk) * E * kSlice * sizeof(float));
+        mbar_arrive_expect_tx(bar, bytes);
+        bulk_g2s(mine, pkp + (int64_t)pk * E * kSlice, bytes, bar, pf);
+        pk += C;
+        if (pk >= pw)
+        {
+            psl += 32;
+            if (psl >= s1)
+                psl = s0 + warp;
+            slice_of();
+        }
+    };
+    if (has && lane == 0)
+    {
+        slice_of();
+        issue();
+    }
+    uint32_t parity = 0;
+    bool dead = false; // a copy did not come in time: nothing more is used or fetched
+
+    double loc = 0;
+    for (int64_t k = gt; k < s.ndof; k += T)
+    {
+        const float v = b[k];
+        st_keep(r + k, v, pl);
+        st_keep(x + k, 0.0f, pl);
+        st_keep(pa + k, 0.0f, pl);
+        loc += (double)v * (double)v;
+    }
+    unsigned epoch = 0;
+    double rr = 0.0, stop = 0.0;
+    bool go = grid_sum(loc, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, s.wait_ns);
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    if (go)
+    {
+        stop = (s.abs_stop >= 0) ? s.abs_stop : s.rtol * rr + s.atol;
+        if (lead)
+        {
+            s.info[0] = 0;
+            reinterpret_cast<double *>(s.info)[2] = rr;
+            reinterpret_cast<double *>(s.info)[3] = rr;
+        }
+        go = !(rr <= stop);
+    }
+    float beta = 0.0f;
+    float *pold = pa, *pnew = pb;
+    for (int64_t it = 1; go; ++it)
+    {
+        double lpq = 0.0;
+        for (int sl = s0 + warp; sl < s1 && !dead; sl += 32)
+        {
+            const int pos = sl * kSlice + lane;
+            const int i = pos < s.n ? s.perm[pos] : -1;
+            const int myn = i >= 0 ? s.rowptr[i + 1] - s.rowptr[i] : 0;
+            const int64_t off = s.slice_off[sl];
+            const int w = (int)(s.slice_off[sl + 1] - off);
+            const int *cp = s.col_sell + off * kSlice + lane;
+            float acc[D] = {0.0f, 0.0f, 0.0f};
+            int jn[C];
+#pragma unroll
+            for (int u = 0; u < C; ++u)
+                jn[u] = u < myn ? ld_stream(cp + u * kSlice, pf) : 0;
+            for (int k = 0; k < w; k += C)
+            {
+                float xv[C][D], pv[C][D];
+#pragma unroll
+                for (int u = 0; u < C; ++u)
+                    if (k + u < myn)
+#pragma unroll
+                        for (int c = 0; c < D; ++c)
+                        {
+                            xv[u][c] = ld_keep(r + (int64_t)jn[u] * D + c, pl);
+                            pv[u][c] = ld_keep(pold + (int64_t)jn[u] * D + c, pl);
+                        }
+#pragma unroll
+                for (int u = 0; u < C; ++u)
+                    jn[u] = k + C + u < myn ? ld_stream(cp + (int64_t)(k + C + u) * kSlice, pf) : 0;
+                if (!mbar_wait_bounded(bar, parity, s.wait_ns))
+                {
+                    atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 2ull);
+                    s_fail = 1;
+                    dead = true;
+                }
+                dead = __any_sync(0xffffffffu, dead);
+                if (dead)
+                    break;
+                const float *kb = mine + lane;
+#pragma unroll
+                for (int u = 0; u < C; ++u)
+                    if (k + u < myn)
+                    {
+#pragma unroll
+                        for (int c = 0; c < D; ++c)
+                            xv[u][c] = xv[u][c] + beta * pv[u][c];
+#pragma unroll
+                        for (int a = 0; a < D; ++a)
+#pragma unroll
+                            for (int c = 0; c < D; ++c)
+                                acc[a] += kb[(u * E + a * D + c) * kSlice] * xv[u][c];
+                    }
+                __syncwarp();
+                if (lane == 0)
+                    issue();
+                parity ^= 1;
+            }
+            if (i >= 0)
+#pragma unroll
+                for (int c = 0; c < D; ++c)
+                {
+                    const int64_t k = (int64_t)i * D + c;
+                    const float pn = ld_keep(r + k, pl) + beta * ld_keep(pold + k, pl);
+                    st_keep(pnew + k, pn, pl);
+                    st_keep(q + k, acc[c], pl);
+                    lpq += (double)pn * (double)acc[c];
+                }
+        }
+        double pq;
+        if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
+            break;
+        if (pq == 0.0)
+        {
+            if (lead)
+            {
+                s.info[0] = it - 1;
+                atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 4ull);
+            }
+            break;
+        }
+        const float al = (float)(rr / pq);
+        double lrr = 0;
+        for (int64_t k = gt; k < s.ndof; k += T)
+        {
+            const float pn = ld_keep(pnew + k, pl);
+            st_keep(x + k, ld_keep(x + k, pl) + al * pn, pl);
+            const float rv = ld_keep(r + k, pl) - al * ld_keep(q + k, pl);
+            st_keep(r + k, rv, pl);
+            lrr += (double)rv * (double)rv;
+        }
+        double rn;
+        if (!grid_sum(lrr, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, s.wait_ns))
+            break;
+        const bool done = rn <= stop;
+        if (done || it >= s.maxit)
+        {
+            if (lead)
+            {
+                s.info[0] = it;
+                reinterpret_cast<double *>(s.info)[3] = rn;
+                if (!done)
+                    atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 1ull);
+            }
+            break;
+        }
+        beta = (float)(rn / rr);
+        rr = rn;
+        float *t = pold;
+        pold = pnew;
+        pnew = t;
+    }
+    // the copy in flight ends before the block's shared memory is given back
+    if (has)
+        mbar_wait_bounded(bar, parity, kBarrierTimeoutNs);
 }
 
 // ---- helpers for the mixed-precision refinement
@@ -307,7 +522,17 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     void *args[] = {&s, &K, &b, &x, &r, &pa, &pb, &q};
     if ((e = cudaEventRecord(p.cg_ev[0], p.stream)) != cudaSuccess)
         return e;
-    e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D>, dim3(grid), dim3(kCGThreads), args, 0, p.stream);
+    // the streamed form where every block has more than half a slice per warp, so no columns are split
+    if (sizeof(TV) == 4 && D == 3 && 2 * (p.nslices / grid) > kCGThreads / 32)
+    {
+        if ((e = cudaFuncSetAttribute(k_cg_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem)) !=
+            cudaSuccess)
+            return e;
+        e = cudaLaunchCooperativeKernel((const void *)k_cg_stream, dim3(grid), dim3(kCGThreads), args, kStreamSmem,
+                                        p.stream);
+    }
+    else
+        e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D>, dim3(grid), dim3(kCGThreads), args, 0, p.stream);
     if (e != cudaSuccess)
         return e;
     p.ctr.kernel_launches++;
