@@ -54,14 +54,32 @@ struct CGState
     double *part;       // [grid][2]
     int64_t *info;      // [0] iterations, [1] status bits (1 maxit, 2 timeout, 4 breakdown), [2..3] rr0/rr bits
     unsigned long long wait_ns; // limit of each grid-barrier wait
+    int steps;          // RES: columns of a warp at most
 };
 
 
-template <typename TK, typename TV, int D>
+// The column split of spmv_block for a block of ns slices: warps per slice.
+__host__ __device__ __forceinline__ int column_split(int ns, int nw)
+{
+    int S = 2;
+    while (S < kMaxColumnSplit && ns * S * 2 <= nw)
+        S *= 2;
+    return S;
+}
+
+// RES: a warp's columns and values are the same in every iteration, so they are copied to shared memory
+// once, and its row and row length stay in registers; per iteration only r and p are read from L2.
+// Otherwise the chain perm -> rowptr -> column -> r, p starts at L2 again after each grid sum, which
+// empties L1.  The sums are spmv_block's, so the bits are too.  us per iteration, without -> with: FP64 hex
+// 18,000 rows 9.30 -> 7.92, 9,000 8.25 -> 7.03, 3,900 7.78 -> 6.58, square 17,550 8.06 -> 6.76; FP32 hex
+// 18,000 8.39 -> 6.96.  What is left is the two grid sums (2.0 us each) and the latency of the gathers.
+// s.steps: the most columns of a warp.
+template <typename TK, typename TV, int D, bool RES>
 __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, const TK *__restrict__ K, const TV *__restrict__ b,
                                                    TV *__restrict__ x, TV *__restrict__ r, TV *__restrict__ pa,
                                                    TV *__restrict__ pb, TV *__restrict__ q)
 {
+    extern __shared__ __align__(16) unsigned char cg_sm[];
     __shared__ double sh[32];
     __shared__ int s_fail;
     __shared__ TV red[32 * D * 32];
@@ -76,6 +94,31 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
     const int s1 = (int)((int64_t)(blockIdx.x + 1) * s.nslices / gridDim.x);
     const int warp = threadIdx.x >> 5;
     const uint64_t pf = l2_evict_first(), pl = l2_evict_last();
+
+    int ri = -1, rn_ = 0, part = 0, split = 1; // RES: the lane's row, its columns here, the warp's part
+    TK *kS = reinterpret_cast<TK *>(cg_sm) + (size_t)warp * s.steps * D * D * kSlice + (threadIdx.x & 31);
+    int *cS = reinterpret_cast<int *>(reinterpret_cast<TK *>(cg_sm) + (size_t)(blockDim.x >> 5) * s.steps * D * D * kSlice) +
+              warp * s.steps * kSlice + (threadIdx.x & 31);
+    if constexpr (RES)
+    {
+        split = column_split(s1 - s0, blockDim.x >> 5);
+        part = warp % split;
+        const int sl = s0 + warp / split, pos = sl * kSlice + (threadIdx.x & 31);
+        if (sl < s1 && pos < s.n)
+        {
+            ri = s.perm[pos];
+            const int myn = s.rowptr[ri + 1] - s.rowptr[ri];
+            const int64_t off = s.slice_off[sl];
+            for (int k = part; k < myn; k += split, ++rn_)
+            {
+                const int64_t at = (off + k) * kSlice + (threadIdx.x & 31);
+                cS[rn_ * kSlice] = s.col_sell[at];
+#pragma unroll
+                for (int e = 0; e < D * D; ++e)
+                    kS[(rn_ * D * D + e) * kSlice] = K[((off + k) * D * D + e) * kSlice + (threadIdx.x & 31)];
+            }
+        }
+    }
 
     double loc = 0;
     for (int64_t k = gt; k < s.ndof; k += T)
@@ -102,8 +145,54 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks) k_cg(CGState s, cons
     TV *pold = pa, *pnew = pb;
     for (int64_t it = 1;; ++it)
     {
-        const double lpq = spmv_block<TK, TV, D>(s0, s1, s.n, s.rowptr, s.perm, s.slice_off, s.col_sell, K, r,
-                                                   pold, pnew, q, beta, pf, pl, red);
+        double lpq = 0.0;
+        if constexpr (RES)
+        {
+            TV acc[D], pn[D];
+#pragma unroll
+            for (int c = 0; c < D; ++c)
+            {
+                acc[c] = TV(0);
+                if (part == 0 && ri >= 0)
+                    pn[c] = ld_keep(r + (int64_t)ri * D + c, pl) + beta * ld_keep(pold + (int64_t)ri * D + c, pl);
+            }
+#pragma unroll 4
+            for (int t = 0; t < rn_; ++t)
+            {
+                const int j = cS[t * kSlice];
+                TV xv[D];
+#pragma unroll
+                for (int c = 0; c < D; ++c)
+                    xv[c] = ld_keep(r + (int64_t)j * D + c, pl) + beta * ld_keep(pold + (int64_t)j * D + c, pl);
+#pragma unroll
+                for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                    for (int c = 0; c < D; ++c)
+                        acc[rr] += kS[(t * D * D + rr * D + c) * kSlice] * xv[c];
+            }
+            if (part > 0)
+#pragma unroll
+                for (int c = 0; c < D; ++c)
+                    red[(warp * D + c) * 32 + (threadIdx.x & 31)] = acc[c];
+            __syncthreads();
+            if (part == 0 && ri >= 0)
+            {
+                for (int p = 1; p < split; ++p)
+#pragma unroll
+                    for (int c = 0; c < D; ++c)
+                        acc[c] += red[((warp + p) * D + c) * 32 + (threadIdx.x & 31)];
+#pragma unroll
+                for (int c = 0; c < D; ++c)
+                {
+                    st_keep(pnew + (int64_t)ri * D + c, pn[c], pl);
+                    st_keep(q + (int64_t)ri * D + c, acc[c], pl);
+                    lpq += (double)pn[c] * (double)acc[c];
+                }
+            }
+        }
+        else
+            lpq = spmv_block<TK, TV, D>(s0, s1, s.n, s.rowptr, s.perm, s.slice_off, s.col_sell, K, r, pold, pnew, q, beta,
+                                        pf, pl, red);
         double pq;
         if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, s.wait_ns))
             return;
@@ -436,7 +525,7 @@ static cudaError_t cg_grid_rule(const Problem &p, int *grid_out)
     int &occ = occ_cache[sizeof(TK) == 8][sizeof(TV) == 8][D];
     if (occ == 0)
     {
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg<TK, TV, D>, kCGThreads, 0);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg<TK, TV, D, false>, kCGThreads, 0);
         if (e != cudaSuccess)
             return e;
         if (occ < 1)
@@ -449,6 +538,25 @@ static cudaError_t cg_grid_rule(const Problem &p, int *grid_out)
         grid = kMaxGridBlocks;
     *grid_out = grid;
     return cudaSuccess;
+}
+
+// k_cg's RES form on `grid` blocks: columns of a warp at most, 0 where it does not serve, which is where
+// a block has more than half a slice per warp or its matrix does not fit (2D FP64: above four slices a
+// block, 18,900 rows).  It is the faster form wherever it fits.
+constexpr size_t kResidentSmem = 176 * 1024;
+template <typename TK, int D>
+static size_t resident_bytes(int steps)
+{
+    return (size_t)(kCGThreads / 32) * steps * kSlice * (D * D * sizeof(TK) + sizeof(int));
+}
+template <typename TK, int D>
+static int resident_steps(const Problem &p, int grid)
+{
+    const int nw = kCGThreads / 32, most = div_up(p.nslices, grid);
+    if (2 * most > nw)
+        return 0;
+    const int steps = div_up(p.max_conns, column_split(most, nw));
+    return resident_bytes<TK, D>(steps) <= kResidentSmem ? steps : 0;
 }
 
 // Waits for the CG launch between the handle's two events and reads its status words.
@@ -515,6 +623,7 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     s.part = p.partials;
     s.info = p.cg_info;
     s.wait_ns = p.wait_ns;
+    s.steps = 0;
     if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), p.stream)) != cudaSuccess)
         return e;
     if ((e = cudaMemsetAsync(p.cg_info, 0, 4 * sizeof(int64_t), p.stream)) != cudaSuccess)
@@ -531,8 +640,19 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
         e = cudaLaunchCooperativeKernel((const void *)k_cg_stream, dim3(grid), dim3(kCGThreads), args, kStreamSmem,
                                         p.stream);
     }
+    else if (resident_steps<TK, D>(p, grid) > 0)
+    {
+        s.steps = resident_steps<TK, D>(p, grid);
+        const size_t smem = resident_bytes<TK, D>(s.steps);
+        if ((e = cudaFuncSetAttribute(k_cg<TK, TV, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess)
+            return e;
+        e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D, true>, dim3(grid), dim3(kCGThreads), args, smem,
+                                        p.stream);
+    }
     else
-        e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D>, dim3(grid), dim3(kCGThreads), args, 0, p.stream);
+        e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D, false>, dim3(grid), dim3(kCGThreads), args, 0,
+                                        p.stream);
     if (e != cudaSuccess)
         return e;
     p.ctr.kernel_launches++;
