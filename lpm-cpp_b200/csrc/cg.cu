@@ -1039,17 +1039,15 @@ struct CGBsr
 };
 
 // One row of q = A (r + beta p_old), by a warp.  The row's blocks are contiguous, so the lanes read
-// its values in order: in 2D lane l holds entry l % 4 of every eighth block, in 3D lane l < 27 entry
-// l % 9 of every third.  kBsrUnroll blocks of a lane are in flight, their columns fetched one group
-// ahead.  Lane c < D returns q's component c.
+// its values in order: lane l holds entry l % 4 of every eighth block.  kBsrUnroll blocks of a lane are in
+// flight, their columns fetched one group ahead.  Lane c < D returns q's component c.
 constexpr int kBsrUnroll = 4;
-template <int D>
 __device__ __forceinline__ double bsr_row(const CGBsr &s, int row, const double *r, const double *pold, double beta,
                                           uint64_t pm, uint64_t pl)
 {
-    constexpr int E = D * D, KB = D == 2 ? 8 : 3;
+    constexpr int D = 2, E = 4, KB = 8;
     const int lane = threadIdx.x & 31, e = lane % E, kb = lane / E, c = e % D;
-    const int end = kb < KB ? s.rowptr[row + 1] : 0;
+    const int end = s.rowptr[row + 1];
     int bk = s.rowptr[row] + kb;
     double acc = 0.0;
     int jn[kBsrUnroll];
@@ -1078,32 +1076,22 @@ __device__ __forceinline__ double bsr_row(const CGBsr &s, int row, const double 
                 acc += v[u] * (xr[u] + beta * xp[u]);
     }
     // entry (i, c) of the KB lanes that share it, then the row i's D entries
-    if constexpr (D == 2)
-    {
-        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        return __shfl_sync(0xffffffffu, acc, (lane & 1) * 2);
-    }
-    else
-    {
-        acc = acc + __shfl_sync(0xffffffffu, acc, (lane + 9) & 31) + __shfl_sync(0xffffffffu, acc, (lane + 18) & 31);
-        acc = acc + __shfl_sync(0xffffffffu, acc, (lane + 1) & 31) + __shfl_sync(0xffffffffu, acc, (lane + 2) & 31);
-        return __shfl_sync(0xffffffffu, acc, (lane % 3) * 3);
-    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    return __shfl_sync(0xffffffffu, acc, (lane & 1) * 2);
 }
 
-// The CG of k_cg on a caller's block-CSR matrix: a warp per row, each block a contiguous share of the
-// rows.  Bound by the latency of the matrix loads (from L2 while it fits) at four blocks in flight
-// per lane, and by the two grid barriers (2.5 us each).  Whole solves: 15,625 rows in 3D (68 MB) 99.3
-// -> 12.4 ms, 1,085 rows in 2D 11.9 -> 1.42 ms; before, a thread had a row (uncoalesced) and a grid
-// one block per 1,024 rows.
-template <int D>
+// The CG of k_cg on a caller's block-CSR matrix in 2D: a warp per row, each block a contiguous share of
+// the rows.  Bound by the two grid sums (2.0 us each) and the latency of the matrix loads (from L2 while
+// it fits) at four blocks in flight per lane.  Serves what does not fit one cluster (cg_cluster.cu): 11,000
+// hexagonal rows 5.7 ms a solve.
 __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
     k_cg_bsr_noalloc(CGBsr s, const double *__restrict__ b, double *__restrict__ x, double *r, double *pa, double *pb,
                      double *q)
 {
+    constexpr int D = 2;
     __shared__ double sh[32];
     __shared__ int s_fail;
     if (threadIdx.x == 0)
@@ -1140,7 +1128,7 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
         double lpq = 0;
         for (int row = row0 + warp; row < row1; row += nw)
         {
-            const double qv = bsr_row<D>(s, row, r, pold, beta, pm, pl);
+            const double qv = bsr_row(s, row, r, pold, beta, pm, pl);
             if (lane < D)
             {
                 const int64_t k = (int64_t)row * D + lane;
@@ -1192,6 +1180,268 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
     }
 }
 
+// 32 blocks of a row at most: row, first block, end of the row's blocks
+struct BsrChunk
+{
+    int row, k, end;
+    __device__ __forceinline__ int count() const { return min(32, end - k); }
+    __device__ __forceinline__ bool last() const { return k + 32 >= end; }
+    // the next chunk of rows [ra, rb), after the last one the first
+    __device__ __forceinline__ BsrChunk next(const int *__restrict__ rowptr, int ra, int rb) const
+    {
+        BsrChunk c = *this;
+        if (last())
+        {
+            const bool wrap = row + 1 >= rb;
+            c.row = wrap ? ra : row + 1;
+            c.k = wrap ? rowptr[ra] : end;
+            c.end = rowptr[c.row + 1];
+        }
+        else
+            c.k += 32;
+        return c;
+    }
+};
+
+// The CG on a caller's block-CSR matrix in 3D.  A block has a contiguous share of the rows, a warp a
+// contiguous share of those, which it walks in chunks of at most 32 blocks of a row, a lane per block.  A
+// chunk's values come by bulk copy into one of the warp's two buffers while the chunk before it is used,
+// its columns a chunk earlier still; both go on over the grid sums, since the matrix stays.  r and p are
+// gathered a chunk ahead in registers.  Bound by the shared-memory and L1 wavefronts of the values (18 a
+// chunk, 8 bytes at a stride of 72) and of the gathers (36), 26,000 -> 20,000 cycles a product of 105 rows
+// per SM.  Whole solves, lanes over a row's entries as in k_cg_bsr_noalloc -> here: SC 15,625 rows (68 MB)
+// 12.3 -> 9.9 ms, SC 1,728 2.5 -> 1.95, FCC 7,488 6.2 -> 5.4, BCC 11,664 7.8 -> 7.4.  Threads 384 / 512 /
+// 640 / 768: 11.8 / 10.0 / 9.9 / 10.3 ms; asynchronous copies by the lanes in place of the bulk copies
+// 10.9; gathers and copies two chunks ahead 10.7.  In 2D, with 8 to 31 blocks a row, a chunk leaves lanes
+// idle: 5,700 -> 6,240 us at 11,000 hexagonal rows, so 2D keeps k_cg_bsr_noalloc.
+constexpr int kBsrThreads = 640;
+constexpr int kBsrBuf = 32 * 9 + 2; // doubles of a chunk and its odd start
+constexpr size_t kBsrSmem = sizeof(double) * 2 * kBsrBuf * (kBsrThreads / 32);
+
+__global__ void __launch_bounds__(kBsrThreads, 1)
+    k_cg_bsr_chunks(CGBsr s, const double *__restrict__ b, double *__restrict__ x, double *r, double *pa, double *pb,
+                    double *q)
+{
+    constexpr int D = 3, E = 9;
+    extern __shared__ __align__(16) double bsr_sm[];
+    __shared__ uint64_t full[2 * (kBsrThreads / 32)];
+    __shared__ double sh[32];
+    __shared__ int s_fail;
+    if (threadIdx.x == 0)
+        s_fail = 0;
+    unsigned epoch = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row0 = (int)((int64_t)blockIdx.x * s.nrows / gridDim.x),
+              row1 = (int)((int64_t)(blockIdx.x + 1) * s.nrows / gridDim.x);
+    const int ra = row0 + (row1 - row0) * warp / (kBsrThreads / 32),
+              rb = row0 + (row1 - row0) * (warp + 1) / (kBsrThreads / 32);
+    double *buf = bsr_sm + 2 * kBsrBuf * warp;
+    uint64_t *bar = full + 2 * warp;
+    if (lane == 0)
+    {
+        mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    const int64_t k0 = (int64_t)row0 * D, k1 = (int64_t)row1 * D;
+    const int64_t bytes = (int64_t)s.rowptr[s.nrows] * (E * 8 + 4);
+    const uint64_t pl = l2_evict_last(), pm = bytes <= ((int64_t)90 << 20) ? pl : l2_evict_first();
+    // the warp's chunks go round its rows: c0 is used next and its copy is in flight, c1 follows it
+    auto phase = [&](const BsrChunk &c) { return (int)((reinterpret_cast<uintptr_t>(s.val + (int64_t)c.k * E) >> 3) & 1); };
+    // the entry of chunk c that this lane fetches by itself (the 16-byte copies leave out odd ends), or -1
+    auto odd_entry = [&](const BsrChunk &c) {
+        const int nd = c.count() * E, ph = phase(c);
+        return lane == 0 ? (ph && nd > 0 ? 0 : -1) : lane == 1 && nd > ph && ((nd - ph) & 1) ? nd - 1 : -1;
+    };
+    double odd = 0.0;
+    auto copy = [&](const BsrChunk &c, int to) {
+        const double *src = s.val + (int64_t)c.k * E;
+        const int ph = phase(c), oe = odd_entry(c), np = c.count() > 0 ? (c.count() * E - ph) >> 1 : 0;
+        if (oe >= 0)
+            odd = ld_stream(src + oe, pm);
+        if (lane == 0)
+        {
+            mbar_arrive_expect_tx(bar + to, (uint32_t)(16 * np));
+            if (np > 0)
+                bulk_g2s(buf + to * kBsrBuf + 2 * ph, src + ph, (uint32_t)(16 * np), bar + to, pm);
+        }
+    };
+    auto column = [&](const BsrChunk &c) { return lane < c.count() ? ld_stream(s.col + c.k + lane, pm) : 0; };
+    BsrChunk c0 = {0, 0, 0}, c1 = c0;
+    int j0 = 0, j1 = 0, flip = 0;
+    unsigned parity = 0; // bit f: the parity that buffer f completes next
+    bool dead = false;   // a copy did not come in time
+    if (ra < rb)
+    {
+        c0 = {ra, s.rowptr[ra], s.rowptr[ra + 1]};
+        copy(c0, 0);
+        c1 = c0.next(s.rowptr, ra, rb);
+        j0 = column(c0);
+        j1 = column(c1);
+    }
+    double loc = 0;
+    for (int64_t k = k0 + threadIdx.x; k < k1; k += blockDim.x)
+    {
+        const double v = b[k];
+        st_keep(r + k, v, pl);
+        x[k] = 0.0;
+        st_keep(pa + k, 0.0, pl);
+        loc += v * v;
+    }
+    double rr = 0.0;
+    bool go = grid_sum(loc, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rr, kBarrierTimeoutNs);
+    const double stop = s.rtol * rr + s.atol;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        s.info[0] = 0;
+    go = go && !(rr <= stop);
+    double beta = 0.0;
+    double *pold = pa, *pnew = pb;
+    for (int64_t it = 1; go; ++it)
+    {
+        double lpq = 0;
+        if (ra < rb && !dead)
+        {
+            double gr[D], gp[D], xv[D], acc[D];
+            auto gather = [&](const BsrChunk &c, int j) {
+                if (lane < c.count())
+#pragma unroll
+                    for (int a = 0; a < D; ++a)
+                    {
+                        gr[a] = ld_keep(r + (int64_t)j * D + a, pl);
+                        gp[a] = ld_keep(pold + (int64_t)j * D + a, pl);
+                    }
+            };
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                gr[a] = gp[a] = acc[a] = 0.0;
+            gather(c0, j0);
+            for (;;)
+            {
+#pragma unroll
+                for (int a = 0; a < D; ++a)
+                    xv[a] = gr[a] + beta * gp[a];
+                const bool more = !(c0.last() && c0.row + 1 >= rb);
+                const double odd0 = odd;
+                copy(c1, flip ^ 1);
+                if (more)
+                    gather(c1, j1);
+                // p of the row, for the lanes that will store it
+                const int comp = lane >> 3;
+                const bool owner = c0.last() && (lane & 7) == 0 && comp < D;
+                const int64_t ok = (int64_t)c0.row * D + comp;
+                double ro = 0.0, po = 0.0;
+                if (owner)
+                {
+                    ro = ld_keep(r + ok, pl);
+                    po = ld_keep(pold + ok, pl);
+                }
+                const BsrChunk c2 = c1.next(s.rowptr, ra, rb);
+                const int j2 = column(c2);
+                if (!mbar_wait_bounded(bar + flip, (parity >> flip) & 1, kBarrierTimeoutNs))
+                    dead = true;
+                dead = __any_sync(0xffffffffu, dead);
+                if (dead)
+                {
+                    atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 2ull);
+                    s_fail = 1;
+                    break;
+                }
+                parity ^= 1 << flip;
+                const int oe = odd_entry(c0);
+                if (oe >= 0)
+                    buf[flip * kBsrBuf + phase(c0) + oe] = odd0;
+                __syncwarp();
+                if (lane < c0.count())
+                {
+                    const double *v = buf + flip * kBsrBuf + phase(c0) + lane * E;
+#pragma unroll
+                    for (int a = 0; a < D; ++a)
+#pragma unroll
+                        for (int e = 0; e < D; ++e)
+                            acc[a] += v[a * D + e] * xv[e];
+                }
+                if (c0.last())
+                {
+                    // sums over the lanes: lane 8 h ends with component h
+                    const bool up = lane & 16, up2 = lane & 8;
+                    double u0 = up ? acc[2] : acc[0], u1 = up ? 0.0 : acc[1];
+                    u0 += __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[2], 16);
+                    u1 += __shfl_xor_sync(0xffffffffu, up ? acc[1] : 0.0, 16);
+                    double t = (up2 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, up2 ? u0 : u1, 8);
+                    t += __shfl_xor_sync(0xffffffffu, t, 4);
+                    t += __shfl_xor_sync(0xffffffffu, t, 2);
+                    t += __shfl_xor_sync(0xffffffffu, t, 1);
+                    if (owner)
+                    {
+                        const double pn = ro + beta * po;
+                        st_keep(pnew + ok, pn, pl);
+                        st_keep(q + ok, t, pl);
+                        lpq += pn * t;
+                    }
+#pragma unroll
+                    for (int a = 0; a < D; ++a)
+                        acc[a] = 0.0;
+                }
+                __syncwarp();
+                c0 = c1;
+                j0 = j1;
+                c1 = c2;
+                j1 = j2;
+                flip ^= 1;
+                if (!more)
+                    break;
+            }
+        }
+        double pq;
+        if (!grid_sum(lpq, s.bar, epoch, s.info, &s_fail, s.part, 1, sh, &pq, kBarrierTimeoutNs))
+            break;
+        if (pq == 0.0)
+        {
+            if (blockIdx.x == 0 && threadIdx.x == 0)
+            {
+                s.info[0] = it - 1;
+                atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 4ull);
+            }
+            break;
+        }
+        const double alpha = rr / pq;
+        double lrr = 0;
+        for (int64_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) // the block's own rows
+        {
+            x[k] = x[k] + alpha * ld_keep(pnew + k, pl);
+            const double rv = ld_keep(r + k, pl) - alpha * ld_keep(q + k, pl);
+            st_keep(r + k, rv, pl);
+            lrr += rv * rv;
+        }
+        double rn;
+        if (!grid_sum(lrr, s.bar, epoch, s.info, &s_fail, s.part, 0, sh, &rn, kBarrierTimeoutNs))
+            break;
+        if (rn <= stop || it >= s.maxit)
+        {
+            if (blockIdx.x == 0 && threadIdx.x == 0)
+            {
+                s.info[0] = it;
+                if (!(rn <= stop))
+                    atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 1ull);
+            }
+            break;
+        }
+        beta = rn / rr;
+        rr = rn;
+        double *t = pold;
+        pold = pnew;
+        pnew = t;
+    }
+    // the copy in flight ends before the block's shared memory is given back
+    if (ra < rb)
+    {
+        mbar_wait_bounded(bar + flip, (parity >> flip) & 1, kBarrierTimeoutNs);
+        if (dead)
+            mbar_wait_bounded(bar + (flip ^ 1), (parity >> (flip ^ 1)) & 1, kBarrierTimeoutNs);
+    }
+}
+
 // The device address of the array in the current device's context, looked up on every call (the
 // lookup allocates nothing): a cached address would dangle after the host application resets the
 // device or re-creates its context, which reloads the module.
@@ -1221,7 +1471,11 @@ static cudaError_t noalloc_launch(double *scr, int grid, const CGBsr &s0, const 
     if (e != cudaSuccess)
         return e;
     void *args[] = {&s, &b, &x, &r, &pa, &pb, &q};
-    e = cudaLaunchCooperativeKernel((const void *)k_cg_bsr_noalloc<D>, dim3(grid), dim3(kCGThreads), args, 0, stream);
+    if constexpr (D == 2)
+        e = cudaLaunchCooperativeKernel((const void *)k_cg_bsr_noalloc, dim3(grid), dim3(kCGThreads), args, 0, stream);
+    else if ((e = cudaFuncSetAttribute(k_cg_bsr_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBsrSmem)) ==
+             cudaSuccess)
+        e = cudaLaunchCooperativeKernel((const void *)k_cg_bsr_chunks, dim3(grid), dim3(kBsrThreads), args, kBsrSmem, stream);
     if (e != cudaSuccess)
         return e;
     e = cudaMemcpyAsync(status, s.info, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, stream);
@@ -1244,24 +1498,21 @@ extern "C" int32_t lpmgpu_cg_bsr_noalloc(int32_t dim, int32_t nrows, const int32
         set_last_error("lpmgpu_cg_bsr_noalloc: more than 262144 unknowns (the size of its static scratch)");
         return LPMGPU_ERR_INVALID_ARG;
     }
-    int dev = 0, sms = 0, occ = 0;
+    int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     double *scr = nullptr;
     if (e == cudaSuccess)
         e = noalloc_scratch(dev, &scr);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = (dim == 2) ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_bsr_noalloc<2>, kCGThreads, 0)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_bsr_noalloc<3>, kCGThreads, 0);
     if (e != cudaSuccess)
     {
         set_last_error(std::string("lpmgpu_cg_bsr_noalloc: ") + cudaGetErrorString(e));
         return e == cudaErrorNoDevice ? LPMGPU_ERR_NO_DEVICE : LPMGPU_ERR_CUDA;
     }
-    int grid = sms * std::max(1, std::min(occ, kCGMinBlocks));
-    grid = std::min(grid, kNoAllocMaxBlocks);
-    grid = std::min(grid, (nrows + kCGThreads / 32 - 1) / (kCGThreads / 32)); // a warp per row
+    const int warps = (dim == 2 ? kCGThreads : kBsrThreads) / 32;
+    int grid = std::min(sms, kNoAllocMaxBlocks); // one block per SM
+    grid = std::min(grid, (nrows + warps - 1) / warps); // a row per warp
     grid = std::max(grid, 1);
     CGBsr s{};
     s.nrows = nrows;
