@@ -329,19 +329,29 @@ __device__ __forceinline__ void general_close(const RowTerms<TV, D> &rt, const T
                          TV(0.25) * (rt.v[2 * D + k] * G0 + rt.v[3 * D + k] * G1));
 }
 
-// The CG on the whole grid, one block per SM, each owning a contiguous share of the groups.  Bound by
-// the bond stream (28 bytes per bond and pass in FP64 3D, twice per iteration, from L2 while it fits
-// there) and its gathers, plus two grid barriers of about 2.5 us.  pq is known after pass 1, so x and r
-// are updated in pass 2 and there is no vector pass.  One bond in flight per lane at 1024 threads: the
-// 64 registers hold no more without spills (two bonds spilled: 70 us per iteration on the cube below;
-// 512 threads with two bonds: 25.1 us).  Measured per iteration against k_cg on the assembled matrix:
-// 51x50x50 simple cubic FP64 98.2 -> 23.1 us (its matrix streams 584 MB at 93% of HBM; its bonds are
-// 64 MB), 125x144 hexagonal FP64 10.2 -> 9.7 us.
-constexpr int kBondThreads = 1024;
+// The CG on the whole grid, one block per SM, each owning a contiguous share of the groups.  pq is known
+// after pass 1, so x and r are updated in pass 2 and there is no vector pass.
+//
+// Large problems: bound by the bond stream (28 bytes per bond and pass in FP64 3D, twice per iteration,
+// from L2 while it fits there) and its gathers, plus two grid sums of 2.0 us.  One bond in flight per lane
+// at 1024 threads: the 64 registers hold no more without spills (two bonds spilled: 70 us per iteration on
+// the cube below; 512 threads with two bonds: 25.1 us against 23.1 then).  51x50x50 simple cubic FP64,
+// assembled matrix (584 MB at 93% of HBM) -> bonds (64 MB): 98.2 -> 20.2 us.
+//
+// ST (uniform coefficients, at most one group per warp, whose bonds fit kStagedSmem): the columns and
+// cosines are copied to shared memory once, since each grid sum empties L1, so a gather no longer waits on
+// a column from L2 and the registers hold three bonds' gathers per lane.  Without -> with ST, us per
+// iteration: hexagonal 18,000 rows 7.76 -> 6.99, 40,000 9.07 -> 8.97, square 21,000 7.19 -> 6.80, simple
+// cubic 8,000 9.06 -> 8.21, 27,000 11.2 -> 9.63, FCC 7,488 9.08 -> 8.43, BCC 16,000 9.01 -> 8.75.  At 1024
+// threads with 1 / 2 / 3 bonds in flight (the latter two spill) hexagonal 18,000 takes 7.38 / 8.25 / 10.2;
+// at 512 with 5, 7.37 and simple cubic 27,000 13.7.
+constexpr int kBondThreads = 1024, kStagedThreads = 512;
+constexpr size_t kStagedSmem = 128 * 1024;
 
-template <typename TV, int D, bool GEN>
-__global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
+template <typename TV, int D, bool GEN, bool ST>
+__global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bond(BondCG<TV> s)
 {
+    extern __shared__ __align__(16) unsigned char bond_sm[];
     __shared__ double sh[32];
     __shared__ int s_fail;
     if (*s.flag & s.flag_bad)
@@ -353,12 +363,37 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
     if (threadIdx.x == 0)
         s_fail = 0;
     __syncthreads();
-    constexpr int U = 1; // bonds in flight per lane
+    constexpr int U = ST ? 3 : 1; // bonds in flight per lane
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n = s.n, ls = s.ls, q = lane & ((1 << ls) - 1), rl = lane >> ls, R = 32 >> ls;
     const int g0 = (int)((int64_t)blockIdx.x * s.ng / gridDim.x), g1 = (int)((int64_t)(blockIdx.x + 1) * s.ng / gridDim.x);
     const uint64_t pl = l2_evict_last(), pb_ = s.keep ? l2_evict_last() : l2_evict_first();
     unsigned epoch = 0;
+    // ST: the bonds of the warp's one group
+    TV *cS = reinterpret_cast<TV *>(bond_sm) + (size_t)warp * s.width * D * 32 + lane;
+    int *colS = reinterpret_cast<int *>(reinterpret_cast<TV *>(bond_sm) + (size_t)(g1 - g0) * s.width * D * 32) +
+                warp * s.width * 32 + lane;
+    if (ST && g0 + warp < g1)
+        for (int t = 0; t < s.width; ++t)
+        {
+            const int64_t at = (int64_t)(g0 + warp) * s.width + t;
+            colS[t * 32] = s.col[at * 32 + lane];
+#pragma unroll
+            for (int k = 0; k < D; ++k)
+                cS[(t * D + k) * 32] = s.c[(at * D + k) * 32 + lane];
+        }
+    const int ts = (g0 + warp) * s.width; // ST: the group's first entry
+    auto column = [&](int t) {
+        if constexpr (ST)
+            return colS[(t - ts) * 32];
+        else
+            return ld_stream(s.col + (int64_t)t * 32 + lane, pb_);
+    };
+    auto staged_cosines = [&](int t, TV *c) {
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+            c[k] = cS[((t - ts) * D + k) * 32];
+    };
 
     double loc = 0;
     for (int g = g0 + warp; g < g1; g += nw)
@@ -415,7 +450,7 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
             int cn[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                cn[u] = (t + u < t1) ? ld_stream(s.col + (int64_t)(t + u) * 32 + lane, pb_) : 0;
+                cn[u] = (t + u < t1) ? column(t + u) : 0;
             for (; t < t1; t += U)
             {
                 int co[U];
@@ -424,7 +459,7 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                 for (int u = 0; u < U; ++u)
                 {
                     co[u] = cn[u];
-                    cn[u] = (t + U + u < t1) ? ld_stream(s.col + (int64_t)(t + U + u) * 32 + lane, pb_) : 0;
+                    cn[u] = (t + U + u < t1) ? column(t + U + u) : 0;
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
@@ -432,10 +467,13 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                     {
                         ld_vec<TV, D>(s.r, n, co[u] >> 1, rv[u], pl);
                         ld_vec<TV, D>(pold, n, co[u] >> 1, pv[u], pl);
-                        const TV *cb = s.c + ((int64_t)(t + u) * D) * 32 + lane;
+                        if constexpr (!ST)
+                        {
+                            const TV *cb = s.c + ((int64_t)(t + u) * D) * 32 + lane;
 #pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            cv[u][k] = ld_stream(cb + k * 32, pb_);
+                            for (int k = 0; k < D; ++k)
+                                cv[u][k] = ld_stream(cb + k * 32, pb_);
+                        }
                         if constexpr (GEN)
                         {
                             T[u] = ld_stream(s.tm + (int64_t)(2 * (t + u)) * 32 + lane, pb_);
@@ -447,6 +485,8 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                     if (t + u < t1)
                     {
                         TV xj[D];
+                        if constexpr (ST)
+                            staged_cosines(t + u, cv[u]);
 #pragma unroll
                         for (int k = 0; k < D; ++k)
                             xj[k] = rv[u][k] + beta * pv[u][k];
@@ -522,7 +562,7 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
             int cn[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                cn[u] = (t + u < t1) ? ld_stream(s.col + (int64_t)(t + u) * 32 + lane, pb_) : 0;
+                cn[u] = (t + u < t1) ? column(t + u) : 0;
             for (; t < t1; t += U)
             {
                 int co[U];
@@ -531,7 +571,7 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                 for (int u = 0; u < U; ++u)
                 {
                     co[u] = cn[u];
-                    cn[u] = (t + U + u < t1) ? ld_stream(s.col + (int64_t)(t + U + u) * 32 + lane, pb_) : 0;
+                    cn[u] = (t + U + u < t1) ? column(t + U + u) : 0;
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
@@ -548,16 +588,21 @@ __global__ void __launch_bounds__(kBondThreads, 1) k_cg_bond(BondCG<TV> s)
                         }
                         else
                             ta[u] = ld_keep(s.th + co[u], pl);
-                        const TV *cb = s.c + ((int64_t)(t + u) * D) * 32 + lane;
+                        if constexpr (!ST)
+                        {
+                            const TV *cb = s.c + ((int64_t)(t + u) * D) * 32 + lane;
 #pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            cv[u][k] = ld_stream(cb + k * 32, pb_);
+                            for (int k = 0; k < D; ++k)
+                                cv[u][k] = ld_stream(cb + k * 32, pb_);
+                        }
                     }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     if (t + u < t1)
                     {
                         const int L = co[u] & 1;
+                        if constexpr (ST)
+                            staged_cosines(t + u, cv[u]);
                         TV w;
                         if constexpr (GEN)
                         {
@@ -1145,9 +1190,19 @@ static int cluster_limit(const Problem &p)
 
 static int groups_of(int n, int ls) { return div_up(n, 32 >> ls); }
 
+// shared memory of the staged grid form on `grid` blocks, and whether that form serves them
+static size_t staged_smem(const Problem &p, int grid, size_t real)
+{
+    return (size_t)div_up(p.bo_ng, grid) * p.bo_width * 32 * (p.dim * real + sizeof(int));
+}
+static bool staged_fits(const Problem &p, int grid, size_t real)
+{
+    return !p.bo_gen && div_up(p.bo_ng, grid) <= kStagedThreads / 32 && staged_smem(p, grid, real) <= kStagedSmem;
+}
+
 // Builds the layout once per problem.  The cluster form when the problem fits one cluster (the grid
 // form's barriers alone cost more than a whole cluster iteration up to that size: 11,500 particles take
-// 5.6 us in a cluster and 9.5 us on the grid), with as many lanes per row as keep a CTA within 8 warps
+// 5.6 us in a cluster and 7.0 us on the grid), with as many lanes per row as keep a CTA within 8 warps
 // of rows (725 particles at 8, 4, 2, 1 lanes: 3.2, 2.9, 2.9, 3.2 us; 4,096 in 3D at 2, 1: 5.9, 5.4 us);
 // else lanes per row so that the grid's threads are used.  Elastic-damage and fatigue particles keep the assembled matrix: their load paths
 // end in torn or unloaded states whose stresses are what the linear solves leave of their rounding.
@@ -1167,8 +1222,18 @@ cudaError_t setup_bond_op(Problem &p)
     int lc = 3, lg = 0; // lanes per row of the cluster form and of the grid form
     while (lc > 0 && div_up(groups_of(p.n, lc), std::max(ncmax, 1)) > 8)
         --lc;
-    while (lg < 2 && ((int64_t)p.n << (lg + 1)) <= (int64_t)p.num_sms * kBondThreads)
-        ++lg;
+    // the grid form: lanes per row so that the staged form's threads are used, where it serves, else the
+    // general one's
+    auto lanes = [&p](int threads) {
+        int l = 0;
+        while (l < 2 && ((int64_t)p.n << (l + 1)) <= (int64_t)p.num_sms * threads)
+            ++l;
+        return l;
+    };
+    lg = lanes(kStagedThreads);
+    shape(lg);
+    if (p.bo_gen || !staged_fits(p, p.num_sms, sizeof(double)))
+        lg = lanes(kBondThreads);
     shape(lc);
     const int G = div_up(p.bo_ng, std::max(ncmax, 1));
     p.bo_nc = (ncmax > 0 && G <= 31 && cluster_smem_of(p, G, G * (32 >> lc)) <= kClusterSmem) ? ncmax : 0;
@@ -1361,7 +1426,7 @@ template <typename TV, int D, bool GEN>
 static cudaError_t bond_grid(const Problem &p, int *grid)
 {
     int occ = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_bond<TV, D, GEN>, kBondThreads, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_bond<TV, D, GEN, false>, kBondThreads, 0);
     if (e != cudaSuccess)
         return e;
     *grid = std::max(1, std::min(p.num_sms * std::min(std::max(occ, 1), 1), p.bo_ng));
@@ -1378,8 +1443,20 @@ static cudaError_t launch_grid(Problem &p, BondCG<TV> &s)
     if (p.cg_grid > 0 && p.cg_grid < grid)
         grid = p.cg_grid;
     void *args[] = {&s};
-    e = cudaLaunchCooperativeKernel((const void *)k_cg_bond<TV, D, GEN>, dim3(grid), dim3(kBondThreads), args, 0,
-                                    p.stream);
+    bool staged = false;
+    if constexpr (!GEN)
+        if (staged_fits(p, grid, sizeof(TV)))
+        {
+            staged = true;
+            if ((e = cudaFuncSetAttribute(k_cg_bond<TV, D, GEN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kStagedSmem)) != cudaSuccess)
+                return e;
+            e = cudaLaunchCooperativeKernel((const void *)k_cg_bond<TV, D, GEN, true>, dim3(grid), dim3(kStagedThreads), args,
+                                            staged_smem(p, grid, sizeof(TV)), p.stream);
+        }
+    if (!staged)
+        e = cudaLaunchCooperativeKernel((const void *)k_cg_bond<TV, D, GEN, false>, dim3(grid), dim3(kBondThreads), args, 0,
+                                        p.stream);
     if (e != cudaSuccess)
         return e;
     p.ctr.kernel_launches++;
