@@ -259,8 +259,8 @@ int32_t lpmgpu_fatigue_cycle(lpmgpu_solver *h, const lpmgpu_load_step *steps, in
 /* Autotuner of the CG launch shape (no counterpart in the reference; the reference's MKL CG has no
  * launch shape).  lpmgpu_autotune re-assembles K from the current state (call it between load
  * steps, after the first, so that the displacement BCs make K definite), then times `iterations` CG iterations of this problem's matrix (the FP32 inner solve in
- * mixed precision) for each candidate grid size: the default (one block per SM, at most one per
- * slice) and 3/4, 1/2, 1/4, 1/8, 1/16 of it.  The fastest stays in force for this handle's later
+ * mixed precision) for each candidate grid size: the default (one block per SM; for a problem that
+ * solves in one cluster, its CTAs) and 3/4, 1/2, 1/4, 1/8, 1/16 of it.  The fastest stays in force for this handle's later
  * solves; results then differ from the default grid's only by the rounding of the reductions.
  * lpmgpu_set_cg_grid sets the grid directly (0 = the default; values above the default are
  * clamped to it). */
@@ -365,7 +365,8 @@ int32_t lpmgpu_cg_bsr_noalloc(int32_t dim, int32_t nrows, const int32_t *rowptr,
  * by the batch) plus its whole load path, copied at lpmgpu_batch_add.  Each member follows
  * exactly the steps of lpmgpu_solve_load_step, load step by load step (halving included); a
  * round advances every member by one piece of device work and solves all members' pending
- * Newton systems in one persistent CG launch.  Members may be added between rounds; finished
+ * Newton systems: those that fit one thread-block cluster each in a cluster of their own, side by
+ * side, the others together in one persistent CG launch.  Members may be added between rounds; finished
  * members may be removed.  A handle must not be used by other calls while it is a running
  * member.  Up to 4096 running members.  Not thread-safe: one host thread per batch. */
 typedef struct lpmgpu_batch lpmgpu_batch;
@@ -386,7 +387,7 @@ typedef struct
     int64_t rounds, cg_launches, members_done, members_failed;
     int64_t cg_iters, dof_iters; /* over members still held by the batch */
     double seconds;              /* wall time inside lpmgpu_batch_run */
-    double cg_kernel_seconds;    /* device time of the batched CG launches */
+    double cg_kernel_seconds;    /* device time of the batched CG launches and the cluster solves */
     int32_t fp32_kernel;         /* the mixed members' CG kernel for launches with at least 8
                                     slices of 32 rows per block: 1, 2 single reduction with 1 or 2 SpMV steps
                                     in flight, 3 single reduction with the matrix streamed into

@@ -18,6 +18,8 @@
 //   * Mixed members run their FP64 refinement inside the launch: x64 += x32, the true FP64
 //     residual and the restart of the next inner FP32 solve, while the others keep iterating.
 //   * All waits are bounded (4 s); a timeout sets a flag and every block returns.
+// Members whose bond form fits one cluster (bond_op.cu) solve alone in theirs instead, many side by
+// side on their own streams; the host takes each result as its flag comes in.
 //
 // Runtime.  Each member follows SolverStatic::solveProblem / solveProblemStep
 // (include/solver_static.h:65-152) exactly as lpmgpu_solve_load_step does: apply the load

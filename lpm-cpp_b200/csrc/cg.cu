@@ -1,6 +1,9 @@
 // Linear solve of the Newton step: the replacement for Solver::LPM_CG (include/solver.h:277-354),
 // i.e. MKL's RCI dcg with mkl_sparse_d_mv on the symmetric upper CSR.
 //
+// Elastic and J2 problems solve on the bond form of K (bond_op.cu), small ones of the other types in one
+// cluster (cg_cluster.cu).  This file routes them and holds the CG on the assembled matrix.
+//
 // One persistent cooperative launch runs the whole unpreconditioned CG (x0 = 0, stop when
 // ||r||^2 <= rtol*||r0||^2 + atol, cap = problem size, the squared-norm test of MKL's dcg with
 // dpar[0] = dpar[1] = 1e-12 set at solver.h:312-313).  Per iteration:
@@ -17,7 +20,8 @@
 // The SpMV runs on the sliced-ELL layout (lpm_internal.cuh): one thread per particle row, a
 // warp per slice of 32 rows.  For block column k every matrix plane load is 256 contiguous
 // bytes (cache-streaming: the matrix is read once per iteration) and the x gathers of the 32
-// rows hit neighbouring particles, so they coalesce and stay in L2 with the vectors.
+// rows hit neighbouring particles, so they coalesce and stay in L2 with the vectors.  k_cg's RES form keeps
+// the matrix in shared memory where it fits; k_cg_stream brings a large FP32 3D matrix there by bulk copies.
 //
 // Mixed precision (LPMGPU_MIXED): the same kernel on an FP32 copy of K with FP32 Krylov
 // vectors (dot products in FP64), inside an FP64 iterative refinement that recomputes the
@@ -841,7 +845,7 @@ cudaError_t solve_linear(Problem &p, CGResult &out)
 
 // ---- autotuner of the CG launch shape (no counterpart in the reference)
 //
-// The persistent CG kernel's cost per iteration is the matrix stream plus two grid barriers.  On
+// A persistent CG's cost per iteration is its matrix or bond stream plus two grid sums (2.0 us each).  On
 // large problems every SM streams and the default grid (one block per SM) is best; on small ones
 // the barriers dominate and fewer, fuller blocks can be faster.  The tuner times `iterations` CG
 // iterations of this problem's own matrix for each candidate grid (the default and its 3/4, 1/2,

@@ -937,8 +937,8 @@ def format_dump(path: str, step: int, box, xyz, xyz_initial, stress, damage, dam
 
 class Batch:
     """Many problems advanced together (lpmgpu_batch_*): each member runs its whole load path
-    as repeated GpuProblem.solve_load_step calls would, and all members' Newton systems of a
-    round go through one persistent CG launch."""
+    as repeated GpuProblem.solve_load_step calls would; the Newton systems of members that fit a
+    thread-block cluster run side by side, the others' go through one persistent CG launch."""
 
     def __init__(self, device: int = 0):
         h = C.c_void_p()
