@@ -396,7 +396,10 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
                     }
                 __syncwarp();
                 if (lane == 0)
+                {
+                    fence_proxy_async_smem(); // the chunk's reads before the copy that overwrites it
                     issue();
+                }
                 parity ^= 1;
             }
             if (i >= 0)
@@ -1266,6 +1269,7 @@ __global__ void __launch_bounds__(kBsrThreads, 1)
             odd = ld_stream(src + oe, pm);
         if (lane == 0)
         {
+            fence_proxy_async_smem(); // the buffer's last use before the copy that overwrites it
             mbar_arrive_expect_tx(bar + to, (uint32_t)(16 * np));
             if (np > 0)
                 bulk_g2s(buf + to * kBsrBuf + 2 * ph, src + ph, (uint32_t)(16 * np), bar + to, pm);
