@@ -257,13 +257,21 @@ struct RowTerms
     }
 };
 
-// what a lane gathers from its bonds in the first pass
-template <typename TV, int D, bool GEN>
+// what a lane gathers from its bonds in the first pass; Z (uniform form): also the part of K x that needs
+// no theta
+template <typename TV, int D, bool GEN, bool Z = false>
 struct Pass1
 {
     TV th0 = TV(0), th1 = TV(0); // theta (GEN: G) per layer
     TV h0 = TV(0), h1 = TV(0);   // GEN: H per layer
     double en = 0.0;             // x . K x's bond terms
+    TV z[D];                     // Z: sum of 2 Kn c d
+    __device__ __forceinline__ Pass1()
+    {
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+            z[k] = TV(0);
+    }
     __device__ __forceinline__ void bond(const TV *xi, const TV *xj, const TV *c, int L, const TV *Kn, TV T, TV M)
     {
         if constexpr (!GEN)
@@ -275,6 +283,13 @@ struct Pass1
             th0 += L ? TV(0) : d;
             th1 += L ? d : TV(0);
             en += (double)(L ? Kn[1] : Kn[0]) * ((double)d * (double)d);
+            if constexpr (Z)
+            {
+                const TV kd = 2 * (L ? Kn[1] : Kn[0]) * d;
+#pragma unroll
+                for (int k = 0; k < D; ++k)
+                    z[k] += c[k] * kd;
+            }
         }
         else
         {
@@ -341,10 +356,13 @@ __device__ __forceinline__ void general_close(const RowTerms<TV, D> &rt, const T
 // ST (uniform coefficients, at most one group per warp, whose bonds fit kStagedSmem): the columns and
 // cosines are copied to shared memory once, since each grid sum empties L1, so a gather no longer waits on
 // a column from L2 and the registers hold three bonds' gathers per lane.  Without -> with ST, us per
-// iteration: hexagonal 18,000 rows 7.76 -> 6.99, 40,000 9.07 -> 8.97, square 21,000 7.19 -> 6.80, simple
-// cubic 8,000 9.06 -> 8.21, 27,000 11.2 -> 9.63, FCC 7,488 9.08 -> 8.43, BCC 16,000 9.01 -> 8.75.  At 1024
+// iteration: hexagonal 18,000 rows 7.76 -> 6.99, 40,000 9.07 -> 8.78, square 21,000 7.19 -> 6.80, simple
+// cubic 8,000 9.06 -> 8.23, 27,000 11.2 -> 9.68, FCC 7,488 9.08 -> 8.17, BCC 16,000 9.01 -> 8.75.  At 1024
 // threads with 1 / 2 / 3 bonds in flight (the latter two spill) hexagonal 18,000 takes 7.38 / 8.25 / 10.2;
-// at 512 with 5, 7.37 and simple cubic 27,000 13.7.
+// at 512 with 5, 7.37 and simple cubic 27,000 13.7.  Its registers also keep z, the part of K p without
+// theta, from pass 1, so pass 2 gathers theta alone: hexagonal 18,000 6.99 -> 6.78, 40,000 8.78 -> 8.61,
+// simple cubic 8,000 8.23 -> 7.72, 27,000 9.68 -> 8.84, FCC 7,488 8.17 -> 7.68.  The general form has no
+// registers for z: it spills, and the cube above goes from 21.2 to 25.9.
 constexpr int kBondThreads = 1024, kStagedThreads = 512;
 constexpr size_t kStagedSmem = 128 * 1024;
 
@@ -432,6 +450,7 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
     {
         // pass 1: p = r + beta p_old on the fly; theta (GEN: alpha, beta) per particle; p . K p
         double lpq = 0;
+        TV zS[D]; // ST: the warp's one group's share of z
         for (int g = g0 + warp; g < g1; g += nw)
         {
             const int i = g * R + rl, ii = min(i, n - 1);
@@ -444,7 +463,7 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
                 for (int k = 0; k < D; ++k)
                     xi[k] = a[k] + beta * b[k];
             }
-            Pass1<TV, D, GEN> ps;
+            Pass1<TV, D, GEN, ST> ps;
             const int t1 = (g + 1) * s.width;
             int t = g * s.width;
             int cn[U];
@@ -495,6 +514,12 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
             }
             const TV a0 = row_sum(ps.th0, ls), a1 = row_sum(ps.th1, ls);
             lpq += ps.en;
+            if constexpr (ST)
+            {
+#pragma unroll
+                for (int k = 0; k < D; ++k)
+                    zS[k] = ps.z[k];
+            }
             if constexpr (GEN)
             {
                 const TV h0 = row_sum(ps.h0, ls), h1 = row_sum(ps.h1, ls);
@@ -555,7 +580,7 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
             }
 #pragma unroll
             for (int k = 0; k < D; ++k)
-                y[k] = TV(0);
+                y[k] = ST ? zS[k] : TV(0);
             Pass1<TV, D, GEN> ps; // GEN: the row's G and H again
             const int t1 = (g + 1) * s.width;
             int t = g * s.width;
@@ -577,7 +602,8 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
                 for (int u = 0; u < U; ++u)
                     if (t + u < t1)
                     {
-                        ld_vec<TV, D>(pnew, n, co[u] >> 1, pv[u], pl);
+                        if constexpr (!ST)
+                            ld_vec<TV, D>(pnew, n, co[u] >> 1, pv[u], pl);
                         if constexpr (GEN)
                         {
                             const auto v = ld_keep2(s.th + 2 * (int64_t)co[u], pl);
@@ -616,6 +642,8 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
                             }
                             w = T[u] * (ta[u] - ci) + tb[u] + M[u] * cj;
                         }
+                        else if constexpr (ST)
+                            w = (L ? s.T[1] : s.T[0]) * (ta[u] + (L ? ti1 : ti0));
                         else
                         {
                             TV d = cv[u][0] * (xi[0] - pv[u][0]);
@@ -697,11 +725,12 @@ __global__ void __launch_bounds__(ST ? kStagedThreads : kBondThreads, 1) k_cg_bo
 // warp owns no rows: it exchanges the sums, p . K p while the others run pass 2 (which needs theta,
 // but alpha only at its end).
 //
-// Bound by latency below about 200 rows per CTA and by shared-memory bandwidth above (20 wavefronts per 32 bonds in 2D and iteration).  Measured per iteration against
-// k_cg on the assembled matrix: hexagonal plates of 725, 2,900 and 11,500 particles 7.9 -> 2.9,
-// 8.3 -> 3.3 and 9.9 -> 5.6 us; simple-cubic cubes of 1,728 and 4,096 particles 9.8 -> 4.1 and
-// 10.6 -> 5.4 us.  Gathering the neighbours from other CTAs' shared memory instead took 4.0, 5.2 and
-// 7.8 us on the plates.
+// Bound by latency below about 200 rows per CTA and by shared-memory bandwidth above.  Pass 1 keeps z in
+// registers, so pass 2 reads theta alone of the partners.  Measured per iteration against k_cg on the
+// assembled matrix: hexagonal plates of 725, 2,900 and 11,500 particles 7.9 -> 2.9, 8.3 -> 3.0 and 9.9 ->
+// 5.2 us; simple-cubic cubes of 1,000 and 4,096 particles 9.8 -> 3.6 and 10.6 -> 4.8 us.  With p gathered
+// again in pass 2: 2.9, 3.5 and 5.75 us on the plates, 3.9 and 5.9 on the cubes.  Gathering the neighbours
+// from other CTAs' shared memory instead took 4.0, 5.2 and 7.8 us on the plates.
 struct ClusterShared
 {
     double part[2][16]; // partial sums of the CTAs: [0] r.r, [1] p.Kp
@@ -914,11 +943,11 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
                 pzS[l] = rzS[h] + beta * pzS[l];
         }
         __syncthreads();
-        double lpq = 0;
+        double lpq = 0, y[D];
         double ti0 = 0.0, ti1 = 0.0, h0 = 0.0, h1 = 0.0;
         if (act)
         {
-            Pass1<double, D, GEN> ps;
+            Pass1<double, D, GEN, !GEN> ps;
 #pragma unroll 2
             for (int e = e0; e < e1; ++e)
             {
@@ -951,6 +980,9 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
             ti0 = row_sum(ps.th0, ls);
             ti1 = row_sum(ps.th1, ls);
             lpq = ps.en;
+#pragma unroll
+            for (int k = 0; k < D; ++k)
+                y[k] = ps.z[k];
             double2 v0 = make_double2(ti0, ti1), v1 = make_double2(0.0, 0.0);
             if constexpr (GEN)
             {
@@ -985,7 +1017,6 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
             cs->sh[1][warp] = lpq;
         ++sec;
         __syncthreads();
-        double y[D];
         if (helper)
         {
             if (lane == 0)
@@ -1000,18 +1031,20 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
                 atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 2ull);
                 atomicMin(&cs->fail, sec);
             }
-#pragma unroll
-            for (int k = 0; k < D; ++k)
-                y[k] = 0.0;
-#pragma unroll 2
+#pragma unroll 4
             for (int e = e0; e < e1; ++e)
             {
                 const unsigned co = colS[e * 32 + lane];
                 const int L = (int)(co & 1u);
                 double c[D], xj[D], w;
-                const double2 pv = pS[co >> 1];
-                xj[0] = pv.x;
-                xj[1] = pv.y;
+                if constexpr (GEN)
+                {
+                    const double2 pv = pS[co >> 1];
+                    xj[0] = pv.x;
+                    xj[1] = pv.y;
+                    if constexpr (D == 3)
+                        xj[2] = pzS[co >> 1];
+                }
                 if constexpr (D == 2)
                 {
                     const double2 cv = reinterpret_cast<const double2 *>(cS)[e * 32 + lane];
@@ -1020,7 +1053,6 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
                 }
                 else
                 {
-                    xj[2] = pzS[co >> 1];
 #pragma unroll
                     for (int k = 0; k < D; ++k)
                         c[k] = cS[(e * D + k) * 32 + lane];
@@ -1041,11 +1073,7 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
                 else
                 {
                     const double tj = reinterpret_cast<const double *>(thS)[co];
-                    double d = c[0] * (p[0] - xj[0]);
-#pragma unroll
-                    for (int k = 1; k < D; ++k)
-                        d += c[k] * (p[k] - xj[k]);
-                    w = (L ? s.T[1] : s.T[0]) * (tj + (L ? ti1 : ti0)) + 2 * (L ? s.Kn[1] : s.Kn[0]) * d;
+                    w = (L ? s.T[1] : s.T[0]) * (tj + (L ? ti1 : ti0));
                 }
 #pragma unroll
                 for (int k = 0; k < D; ++k)
@@ -1202,7 +1230,7 @@ static bool staged_fits(const Problem &p, int grid, size_t real)
 
 // Builds the layout once per problem.  The cluster form when the problem fits one cluster (the grid
 // form's barriers alone cost more than a whole cluster iteration up to that size: 11,500 particles take
-// 5.6 us in a cluster and 7.0 us on the grid), with as many lanes per row as keep a CTA within 8 warps
+// 5.2 us in a cluster and 6.7 us on the grid), with as many lanes per row as keep a CTA within 8 warps
 // of rows (725 particles at 8, 4, 2, 1 lanes: 3.2, 2.9, 2.9, 3.2 us; 4,096 in 3D at 2, 1: 5.9, 5.4 us);
 // else lanes per row so that the grid's threads are used.  Elastic-damage and fatigue particles keep the assembled matrix: their load paths
 // end in torn or unloaded states whose stresses are what the linear solves leave of their rounding.

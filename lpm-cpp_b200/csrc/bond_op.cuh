@@ -7,7 +7,8 @@
 //     theta_i = sum of d_a over i's bonds of the layer   one value per particle and layer
 // the row of particle i is
 //     (K x)_i = sum_a c_a [ T (theta_i + theta_j) + 2 Kn d_a ]
-// and x . K x = sum_i T theta_i^2 + sum_a Kn d_a^2, which is known as soon as theta is.
+// and x . K x = sum_i T theta_i^2 + sum_a Kn d_a^2, which is known as soon as theta is.  The sum of
+// 2 Kn c_a d_a is known then too (z), so the second pass needs only theta_j of the partners.
 //
 // With coefficients that differ from bond to bond (per-bond properties, continuous damage), with
 // T_a = (1 - D_a) Tv_a, F_a = (1 - D_a)(2 Kn_a + Tv_a) equal for a bond and its opposite, S and U the
