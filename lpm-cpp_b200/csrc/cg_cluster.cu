@@ -10,6 +10,7 @@
 
 #include "cg_cluster.cuh"
 #include "cluster.cuh"
+#include "shares.cuh"
 
 namespace lpm
 {
@@ -73,12 +74,17 @@ constexpr int kMaxCtas = 16;
 // slice, part t taking its block columns t, t + 16, ..., and the 16 partial rows are added in order; a
 // slice's p.q is a block's partial; r.r is summed over 32 consecutive unknowns, 32 of those, and blocks.
 // Every value is formed by the same operations in the same order, so the solve keeps its bits.
+//
+// Every CTA has slices (shares.cuh), which is what orders the exchanges: a CTA stores into another's pq, g
+// and r and counts bytes on its mbarriers only after that CTA's own slices' sums of the phase before, so
+// none is ever a phase behind what arrives.
+//
 // Bound by shared-memory bandwidth (the product reads 36 bytes per block, its 16 partial rows go
 // through memory, p and r are whole vectors) and by 60 cycles per level of each warp sum.  A plate of
 // 1,840 particles: 7.3 us per iteration on the grid, 5.7 here.
 struct SellCG
 {
-    int n, nslices, per, width; // slices per CTA, most block columns of a slice
+    int n, nslices, per, width; // most slices of a CTA, most block columns of a slice
     const int *rowptr, *perm, *iperm, *col;
     const int64_t *slice_off;
     const double *K, *b;
@@ -172,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_sell_cluster(SellCG s)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const unsigned nc = gridDim.x, rank = blockIdx.x; // the grid is one cluster
     const int rows = s.nslices * 32, ndof = 2 * s.n;
-    const int sl0 = min(s.nslices, (int)rank * s.per), sl1 = min(s.nslices, sl0 + s.per), ns = sl1 - sl0;
+    const int sl0 = share_begin(s.nslices, nc, rank), ns = share_begin(s.nslices, nc, rank + 1) - sl0;
     // shared memory: the slices' blocks, r (whose place the partial rows take during the product), p,
     // the blocks' columns, each particle's position
     const size_t red_bytes = (size_t)s.per * kSellParts * 64 * 8, vec_bytes = (size_t)rows * 16;
@@ -347,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_sell_cluster(SellCG s)
         __syncthreads();
         if (warp == 0)
         {
-            if (ns > 0 && lane < (int)nc && lane != (int)rank)
+            if (lane < (int)nc && lane != (int)rank)
                 push_bulk(r + 64 * sl0, lane, barR, 512u * ns);
             __syncwarp();
             if (!__all_sync(0xffffffffu, cluster_wait(barR, par, s.wait_ns)) && lane == 0)
@@ -403,7 +409,7 @@ bool sell_cluster_fits(const Problem &p)
     const int nc = sell_ctas();
     if (p.dim != 2 || nc < 1 || p.cg_grid > 0 || p.nslices > std::min(kSellMaxSlices, p.num_sms) || p.n > 0xffff)
         return false;
-    return sell_smem(p.nslices, div_up(p.nslices, nc), p.max_conns) <= kClusterSmem;
+    return sell_smem(p.nslices, share_most(p.nslices, share_ctas(p.nslices, nc)), p.max_conns) <= kClusterSmem;
 }
 
 cudaError_t enqueue_sell_cluster(Problem &p, const double *b, double *x, double rtol, double atol, double abs_stop,
@@ -413,10 +419,10 @@ cudaError_t enqueue_sell_cluster(Problem &p, const double *b, double *x, double 
     if (e != cudaSuccess)
         return e;
     SellCG s;
-    const int nc = sell_ctas();
+    const int nc = share_ctas(p.nslices, sell_ctas());
     s.n = p.n;
     s.nslices = p.nslices;
-    s.per = div_up(p.nslices, nc);
+    s.per = share_most(p.nslices, nc);
     s.width = p.max_conns;
     s.rowptr = p.cstart;
     s.perm = p.perm;
