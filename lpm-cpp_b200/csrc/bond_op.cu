@@ -1152,6 +1152,8 @@ __global__ void __launch_bounds__(1024, 1) k_cg_bond_cluster(BondCG<double> s, i
 #pragma unroll
         for (int k = 0; k < D; ++k)
             s.x[(int64_t)i * D + k] = x[k];
+    if (!ok)
+        drain_pushes();
     cluster_sync(); // no CTA leaves while another may still push into its shared memory
 }
 

@@ -384,6 +384,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_sell_cluster(SellCG s)
     }
     if (sh->fail && threadIdx.x == 0)
         atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 2ull);
+    if (sh->fail)
+        drain_pushes();
     if (oi >= 0)
     {
         s.x[2 * (int64_t)oi] = xv[0];
@@ -653,6 +655,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_cluster(BsrCG s)
     }
     for (int k = threadIdx.x; k < ns * D; k += blockDim.x)
         s.x[a0 * D + k] = xs[k];
+    if (sh->fail)
+        drain_pushes();
     cluster_sync();
     if (sh->fail && threadIdx.x == 0)
         atomicOr(reinterpret_cast<unsigned long long *>(s.info + 1), 2ull);

@@ -1,0 +1,59 @@
+"""The time limits of the device-side waits, form by form.
+
+Each form of the linear solve runs with a limit of 1 ns, which its first exchange, grid sum or copy
+outlasts, and must report LPMGPU_ERR_TIMEOUT; with the default limit back, the same handle must give the
+bits of a handle that never failed.  The forms: the bond CG in one cluster, staged and general on the
+grid; the assembled CG in one cluster, resident, general (FP64 and FP32) and streamed.  No fault, trap or
+endless loop is involved: a wait that passes its limit ends the kernel."""
+import numpy as np
+import pytest
+
+from _util import LPM
+from test_bond_form import TIGHT, _block, _moved
+
+L = LPM.LatticeType
+# lattice, size, exact assembly, precision, slices per block (0: the default grid)
+FORMS = {
+    "bond_cluster_2d": (L.Hexagon2D, 4.0, False, 0, 0),
+    "bond_cluster_3d": (L.SimpleCubic3D, 2.4, False, 0, 0),
+    "bond_staged": (L.Hexagon2D, 25.0, False, 0, 0),
+    "bond_general": (L.SimpleCubic3D, 14.4, False, 0, 0),
+    "assembled_cluster": (L.Hexagon2D, 4.0, True, 0, 0),
+    "assembled_resident": (L.Hexagon2D, 14.3, True, 0, 0),
+    "assembled_general": (L.SimpleCubic3D, 8.4, True, 0, 0),
+    "assembled_fp32": (L.SimpleCubic3D, 8.4, True, 1, 0),
+    "assembled_streamed": (L.SimpleCubic3D, 8.4, True, 1, 17),
+}
+
+
+def _system(case, exact, precision, grid):
+    g = LPM.GpuProblem(case.assembly(), precision=LPM.Precision(precision), **TIGHT)
+    g.set_assembly_exact(exact)
+    g.set_cg_grid(grid)
+    g.apply_load_step(case.load_step(0))
+    g.set_xyz(_moved(case))
+    g.update_force_state()
+    g.assemble(True)
+    g.update_rr()
+    return g
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", list(FORMS))
+def test_limit_is_reported_and_the_handle_recovers(form):
+    lattice, size, exact, precision, per_block = FORMS[form]
+    case = _block(lattice, size)
+    grid = max(1, case.n // 32 // per_block) if per_block else 0
+    ref = _system(case, exact, precision, grid)
+    want, _ = ref.solve_linear()
+    ref.close()
+    g = _system(case, exact, precision, grid)
+    g.set_wait_limit_ns(1)
+    for _ in range(3):
+        with pytest.raises(LPM.LpmGpuError) as ex:
+            g.solve_linear()
+        assert ex.value.status == LPM.ERR_TIMEOUT, str(ex.value)
+    g.set_wait_limit_ns(0)
+    got, st = g.solve_linear()
+    assert st["cg_iters"] > 0 and np.array_equal(got, want)
+    g.close()
