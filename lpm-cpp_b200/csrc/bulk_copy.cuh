@@ -51,6 +51,26 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                  : "memory");
 }
 
+// The refill of a buffer that the block has read: `bytes` from global src to dst, announced and counted on
+// bar's current phase.  The calling thread has synchronised with the buffer's readers; the fence puts
+// their reads before the copy.
+__device__ __forceinline__ void bulk_refill(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    fence_proxy_async_smem();
+    mbar_arrive_expect_tx(bar, bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_refill(void *dst, const void *src, uint32_t bytes, uint64_t *bar, uint64_t pol)
+{
+    fence_proxy_async_smem();
+    mbar_arrive_expect_tx(bar, bytes);
+    if (bytes > 0)
+        bulk_g2s(dst, src, bytes, bar, pol);
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;

@@ -295,8 +295,7 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
     };
     auto issue = [&]() {
         const uint32_t bytes = (uint32_t)(min(C, pw - pk) * E * kSlice * sizeof(float));
-        mbar_arrive_expect_tx(bar, bytes);
-        bulk_g2s(mine, pkp + (int64_t)pk * E * kSlice, bytes, bar, pf);
+        bulk_refill(mine, pkp + (int64_t)pk * E * kSlice, bytes, bar, pf);
         pk += C;
         if (pk >= pw)
         {
@@ -396,10 +395,7 @@ __global__ void __launch_bounds__(kCGThreads, kCGMinBlocks)
                     }
                 __syncwarp();
                 if (lane == 0)
-                {
-                    fence_proxy_async_smem(); // the chunk's reads before the copy that overwrites it
                     issue();
-                }
                 parity ^= 1;
             }
             if (i >= 0)
@@ -1268,12 +1264,7 @@ __global__ void __launch_bounds__(kBsrThreads, 1)
         if (oe >= 0)
             odd = ld_stream(src + oe, pm);
         if (lane == 0)
-        {
-            fence_proxy_async_smem(); // the buffer's last use before the copy that overwrites it
-            mbar_arrive_expect_tx(bar + to, (uint32_t)(16 * np));
-            if (np > 0)
-                bulk_g2s(buf + to * kBsrBuf + 2 * ph, src + ph, (uint32_t)(16 * np), bar + to, pm);
-        }
+            bulk_refill(buf + to * kBsrBuf + 2 * ph, src + ph, (uint32_t)(16 * np), bar + to, pm);
     };
     auto column = [&](const BsrChunk &c) { return lane < c.count() ? ld_stream(s.col + c.k + lane, pm) : 0; };
     BsrChunk c0 = {0, 0, 0}, c1 = c0;

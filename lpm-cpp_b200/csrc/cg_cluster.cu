@@ -564,6 +564,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_cluster(BsrCG s)
     cluster_sync();
     unsigned par0 = 0, par1 = 0;
     auto none = [](unsigned) {};
+    // the sum of p.q tells the others that r may be overwritten: its reads come before their copies
+    auto read = [](unsigned) { fence_async(); };
     bsr_exchange(sh, nc, rank, 0, par0, 0u, loc, none);
     par0 ^= 1;
     double rr = sh->tot[0];
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_cluster(BsrCG s)
                 lpq += p[(a0 + row) * D + lane] * acc;
             }
         }
-        bsr_exchange(sh, nc, rank, 1, par1, 0u, lpq, none);
+        bsr_exchange(sh, nc, rank, 1, par1, 0u, lpq, read);
         par1 ^= 1;
         const double pq = sh->tot[1];
         if (sh->fail)

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "band_chol.cuh"
+#include "bulk_copy.cuh"
 #include "cg_device.cuh"
 
 namespace lpm
@@ -448,16 +449,16 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
     __shared__ double M[32][33]; // M[j][i]: column j, row i of the block, over the diagonal entry j
     __shared__ double inv[32], s[32];
     __shared__ int lost; // a copy did not arrive in time
-    __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ uint64_t bar[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t nblk = (n + kBandNB - 1) / kBandNB;
     if (threadIdx.x == 0)
     {
         lost = 0;
         for (int k = 0; k < 2; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&bar[k])) : "memory");
+            mbar_init(&bar[k], 1);
+        mbar_init_fence();
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     // the copies run through blocks 0 .. nblk - 1, then back to 0; copy q goes to buffer q % 2
     auto block_of = [&](int64_t q) { return q < nblk ? q : 2 * nblk - 1 - q; };
@@ -467,12 +468,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
         const int64_t j0 = block_of(q) * kBandNB, jb = min((int64_t)kBandNB, n - j0);
         // whole 16-byte pieces; the allocation has one spare entry behind an odd last column
         const unsigned bytes = (unsigned)((jb * ldab * 8 + 15) / 16 * 16);
-        const unsigned b = (unsigned)__cvta_generic_to_shared(&bar[q & 1]);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(dsm + (q & 1) * kSolvePanelBytes);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                     "l"(AB + j0 * ldab), "r"(bytes), "r"(b)
-                     : "memory");
+        bulk_refill(dsm + (q & 1) * kSolvePanelBytes, AB + j0 * ldab, bytes, &bar[q & 1]);
     };
     // column j of block q, entry (i, j) at [i - j]
     auto column = [&](int64_t q, int64_t j0, int j) -> const double * {
