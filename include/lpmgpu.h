@@ -275,9 +275,9 @@ typedef struct
 } lpmgpu_tune_result;
 int32_t lpmgpu_autotune(lpmgpu_solver *h, int32_t iterations, lpmgpu_tune_result *out);
 int32_t lpmgpu_set_cg_grid(lpmgpu_solver *h, int32_t grid);
-/* Time limit of each grid-barrier wait inside this handle's CG kernel (default 4 s; ns <= 0
- * restores it).  A wait that exceeds it makes every block of the launch return and the solve
- * report LPMGPU_ERR_TIMEOUT; the handle stays usable.  Its use is testing that path: a limit
+/* Time limit of each wait inside this handle's CG and direct-solve kernels (grid barriers, cluster
+ * exchanges, asynchronous copies; default 4 s; ns <= 0 restores it).  A wait that exceeds it makes
+ * every block of the launch return and the solve report LPMGPU_ERR_TIMEOUT; the handle stays usable.  Its use is testing that path: a limit
  * below the natural barrier wait makes the next solve time out.  No counterpart in the reference,
  * whose CG (MKL dcg, solver.h:303-344) has no device waits. */
 int32_t lpmgpu_set_wait_limit_ns(lpmgpu_solver *h, int64_t ns);

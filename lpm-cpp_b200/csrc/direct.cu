@@ -23,6 +23,7 @@
 #include "band_chol.cuh"
 #include "bulk_copy.cuh"
 #include "cg_device.cuh"
+#include "cluster.cuh"
 
 namespace lpm
 {
@@ -156,7 +157,8 @@ constexpr int kFactorWarps = kFactorThreads / 32;
 
 // All blocks of the cooperative launch: a counting barrier in global memory (bounded: false and
 // *fail = -1 once a wait passed the limit).
-__device__ __forceinline__ bool factor_barrier(unsigned *bar, unsigned &epoch, int *fail, int *s_stop)
+__device__ __forceinline__ bool factor_barrier(unsigned *bar, unsigned &epoch, int *fail, int *s_stop,
+                                               unsigned long long wait_ns)
 {
     __syncthreads();
     if (threadIdx.x == 0)
@@ -166,7 +168,7 @@ __device__ __forceinline__ bool factor_barrier(unsigned *bar, unsigned &epoch, i
         const unsigned target = (epoch + 1u) * gridDim.x;
         const unsigned long long t0 = gtimer();
         while ((int)(ld_acquire(bar) - target) < 0)
-            if (gtimer() - t0 > kBarrierTimeoutNs)
+            if (gtimer() - t0 > wait_ns)
             {
                 atomicExch(fail, -1);
                 *s_stop = 1;
@@ -233,7 +235,8 @@ __device__ __forceinline__ int factor_block(double *v, double (*L)[kLRow], doubl
 }
 
 __global__ void __launch_bounds__(kFactorThreads, 1) k_band_factor(double *AB, int64_t ldab, int64_t kd, int64_t n,
-                                                                  int *fail, unsigned *bar)
+                                                                  int *fail, unsigned *bar,
+                                                                  unsigned long long wait_ns)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
     double(*Lb)[32][kLRow] = reinterpret_cast<double(*)[32][kLRow]>(fsm); // this block's factor and the next one's
@@ -299,7 +302,7 @@ __global__ void __launch_bounds__(kFactorThreads, 1) k_band_factor(double *AB, i
                 if (i0 + u < end && lane < jb && i0 + u - (j0 + lane) <= kd)
                     col[i0 + u] = x[u];
         }
-        if (!factor_barrier(bar, epoch, fail, &s_stop))
+        if (!factor_barrier(bar, epoch, fail, &s_stop, wait_ns))
             return;
         // the factor takes the block's place (every CTA has long read it)
         if (blockIdx.x == gridDim.x - 1 && warp == kFactorWarps - 1 && lane < jb)
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(kFactorThreads, 1) k_band_factor(double *AB, i
                         }
             }
         }
-        if (!factor_barrier(bar, epoch, fail, &s_stop))
+        if (!factor_barrier(bar, epoch, fail, &s_stop, wait_ns))
             return;
     }
 }
@@ -443,7 +446,7 @@ static_assert(2 * kSolvePanelBytes + 12 * 1024 <= 232448, "shared memory of the 
 // copied there ahead of their use; wider bands are read from global memory.
 template <bool PANEL>
 __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *AB, int64_t ldab, int64_t kd, int64_t n,
-                                                                double *y)
+                                                                double *y, int *fail, unsigned long long wait_ns)
 {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ double M[32][33]; // M[j][i]: column j, row i of the block, over the diagonal entry j
@@ -478,16 +481,25 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
     auto arrive = [&](int64_t q) {
         if (!PANEL)
             return;
-        const unsigned b = (unsigned)__cvta_generic_to_shared(&bar[q & 1]), parity = (unsigned)((q >> 1) & 1);
-        const unsigned long long t0 = gtimer();
-        unsigned done = 0;
-        while (!done && gtimer() - t0 < kBarrierTimeoutNs)
-            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                         : "=r"(done)
-                         : "r"(b), "r"(parity)
-                         : "memory");
-        if (!done)
+        const uint32_t parity = (uint32_t)((q >> 1) & 1);
+        // a try may sleep past a limit below 100 us, which cluster_wait minds
+        if (!(wait_ns >= 100000ull ? mbar_wait_bounded(&bar[q & 1], parity, wait_ns)
+                                   : cluster_wait(smem_u32(&bar[q & 1]), parity, wait_ns)))
             lost = 1;
+    };
+    // After the block synchronisation that follows arrive(q): a copy that did not come in time ends the
+    // kernel, and the host learns of it.  The copies in flight, q and q + 1, land before the block's shared
+    // memory is given back.
+    auto given_up = [&](int64_t q) {
+        if (!PANEL || !lost)
+            return false;
+        if (threadIdx.x == 0)
+        {
+            for (int64_t w = q; w < min(q + 2, 2 * nblk); ++w)
+                cluster_wait(smem_u32(&bar[w & 1]), (unsigned)((w >> 1) & 1), kBarrierTimeoutNs);
+            *fail = -1;
+        }
+        return true;
     };
     auto stage = [&](int64_t q, int64_t j0, int jb, bool transposed) { // warp w: column w
         const double v = (warp < jb && lane < jb && lane >= warp && lane - warp <= kd) ? column(q, j0, warp)[lane - warp]
@@ -512,6 +524,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
         arrive(q);
         stage(q, j0, jb, false);
         __syncthreads();
+        if (given_up(q))
+            return;
         if (warp == 0)
         {
             double v = lane < jb ? y[j0 + lane] : 0.0;
@@ -565,6 +579,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
                 s[warp] = y[j] - t0;
         }
         __syncthreads();
+        if (given_up(q))
+            return;
         if (warp == 0)
         {
             // M[j][i] = L(j, i): x_i = (s_i - sum_{j > i} L(j, i) x_j) / L(i, i)
@@ -583,8 +599,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_band_solve(const double *A
         __syncthreads();
         fetch(q + 2);
     }
-    if (lost && threadIdx.x == 0)
-        y[0] = nan(""); // no solution passes for one
 }
 
 // y[d*rank(i)+r] = src[d*i+r]  /  dst[d*i+r] = y[d*rank(i)+r]
@@ -670,7 +684,8 @@ static cudaError_t factor(Problem &p)
     int64_t ld = ldab, k = kd, nn = ndof;
     int *fail = p.band_fail;
     unsigned *bar = p.barrier;
-    void *args[] = {&ab, &ld, &k, &nn, &fail, &bar};
+    unsigned long long wait_ns = p.wait_ns;
+    void *args[] = {&ab, &ld, &k, &nn, &fail, &bar, &wait_ns};
     e = cudaLaunchCooperativeKernel((const void *)k_band_factor, dim3(p.num_sms), dim3(kFactorThreads), args,
                                     kFactorSmem, p.stream);
     p.ctr.kernel_launches++;
@@ -691,10 +706,12 @@ static cudaError_t substitute(Problem &p)
                                                    2 * kSolvePanelBytes);
         if (e != cudaSuccess)
             return e;
-        k_band_solve<true><<<1, kSolveThreads, 2 * kSolvePanelBytes, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y);
+        k_band_solve<true><<<1, kSolveThreads, 2 * kSolvePanelBytes, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y,
+                                                                              p.band_fail, p.wait_ns);
     }
     else
-        k_band_solve<false><<<1, kSolveThreads, 0, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y);
+        k_band_solve<false><<<1, kSolveThreads, 0, p.stream>>>(p.band_ab, ldab, kd, ndof, p.band_y, p.band_fail,
+                                                               p.wait_ns);
     p.ctr.kernel_launches++;
     k_band_perm<<<nb, 256, 0, p.stream>>>(p.n, D, p.band_rank, p.band_y, p.x, 1);
     p.ctr.kernel_launches++;
@@ -737,10 +754,21 @@ int32_t solve_direct(Problem &p)
         p.band_factored = p.k_version;
     }
     e = p.dim == 2 ? substitute<2>(p) : substitute<3>(p);
+    int *fail = reinterpret_cast<int *>(p.cg_info_host + 6);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(fail, p.band_fail, sizeof(int), cudaMemcpyDeviceToHost, p.stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(p.stream);
     if (e != cudaSuccess)
     {
         set_last_error(std::string("direct solver: ") + cudaGetErrorString(e));
         return LPMGPU_ERR_CUDA;
+    }
+    if (*fail)
+    {
+        p.band_factored = -1; // the next call starts from the band
+        set_last_error("direct solver: a device-side copy wait of the substitution timed out");
+        return LPMGPU_ERR_TIMEOUT;
     }
     return LPMGPU_OK;
 }

@@ -860,7 +860,7 @@ class GpuProblem:
         _check(lib().lpmgpu_set_assembly_exact(self._h, int(bool(exact))), "lpmgpu_set_assembly_exact")
 
     def set_wait_limit_ns(self, ns: int):
-        """Time limit of each grid-barrier wait in this problem's CG kernel; 0 restores the
+        """Time limit of each wait in this problem's CG and direct-solve kernels; 0 restores the
         default of 4 s (lpmgpu_set_wait_limit_ns).  A solve whose wait exceeds it raises
         LpmGpuError with LPMGPU_ERR_TIMEOUT, and the problem stays usable."""
         _check(lib().lpmgpu_set_wait_limit_ns(self._h, int(ns)), "lpmgpu_set_wait_limit_ns")

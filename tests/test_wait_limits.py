@@ -3,8 +3,9 @@
 Each form of the linear solve runs with a limit of 1 ns, which its first exchange, grid sum or copy
 outlasts, and must report LPMGPU_ERR_TIMEOUT; with the default limit back, the same handle must give the
 bits of a handle that never failed.  The forms: the bond CG in one cluster, staged and general on the
-grid; the assembled CG in one cluster, resident, general (FP64 and FP32) and streamed.  No fault, trap or
-endless loop is involved: a wait that passes its limit ends the kernel."""
+grid; the assembled CG in one cluster, resident, general (FP64 and FP32) and streamed; the direct solve's
+factorisation and substitution.  No fault, trap or endless loop is involved: a wait that passes its limit
+ends the kernel."""
 import numpy as np
 import pytest
 
@@ -56,4 +57,24 @@ def test_limit_is_reported_and_the_handle_recovers(form):
     g.set_wait_limit_ns(0)
     got, st = g.solve_linear()
     assert st["cg_iters"] > 0 and np.array_equal(got, want)
+    g.close()
+
+
+@pytest.mark.gpu
+def test_direct_solve():
+    """The factorisation's grid barriers, then the copies of the substitution on a factor that exists."""
+    case = _block(L.Hexagon2D, 6.0)
+    ref = _system(case, False, 0, 0)
+    want, _ = ref.solve_direct()
+    ref.close()
+    g = _system(case, False, 0, 0)
+    for _ in range(2):  # without a factor, then with one
+        g.set_wait_limit_ns(1)
+        for _ in range(2):
+            with pytest.raises(LPM.LpmGpuError) as ex:
+                g.solve_direct()
+            assert ex.value.status == LPM.ERR_TIMEOUT, str(ex.value)
+        g.set_wait_limit_ns(0)
+        got, _ = g.solve_direct()
+        assert np.array_equal(got, want)
     g.close()
