@@ -558,15 +558,13 @@ cudaError_t launch_assemble(Problem &p, bool apply_bc, bool *k32_written)
     const int threads = std::min(256, std::max(32, ((p.max_conns + 31) / 32) * 32));
     if (p.dim == 2)
     {
-        if ((e = cudaFuncSetAttribute(k_assemble<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        if ((e = allow_dynamic_smem((const void *)k_assemble<2>)) != cudaSuccess)
             return e;
         k_assemble<2><<<p.n, threads, smem, p.stream>>>(a);
     }
     else
     {
-        if ((e = cudaFuncSetAttribute(k_assemble<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        if ((e = allow_dynamic_smem((const void *)k_assemble<3>)) != cudaSuccess)
             return e;
         k_assemble<3><<<p.n, threads, smem, p.stream>>>(a);
     }

@@ -586,15 +586,13 @@ cudaError_t launch_assemble_fast(Problem &p, bool apply_bc, bool write_k32)
     const int grid = div_up(p.n, kAsmWarps);
     if (p.dim == 2)
     {
-        if ((e = cudaFuncSetAttribute(k_assemble_fast<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        if ((e = allow_dynamic_smem((const void *)k_assemble_fast<2>)) != cudaSuccess)
             return e;
         k_assemble_fast<2><<<grid, 32 * kAsmWarps, smem, p.stream>>>(a);
     }
     else
     {
-        if ((e = cudaFuncSetAttribute(k_assemble_fast<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        if ((e = allow_dynamic_smem((const void *)k_assemble_fast<3>)) != cudaSuccess)
             return e;
         k_assemble_fast<3><<<grid, 32 * kAsmWarps, smem, p.stream>>>(a);
     }

@@ -546,7 +546,6 @@ static cudaError_t cg_grid_rule(const Problem &p, int *grid_out)
 // k_cg's RES form on `grid` blocks: columns of a warp at most, 0 where it does not serve, which is where
 // a block has more than half a slice per warp or its matrix does not fit (2D FP64: above four slices a
 // block, 18,900 rows).  It is the faster form wherever it fits.
-constexpr size_t kResidentSmem = 176 * 1024;
 template <typename TK, int D>
 static size_t resident_bytes(int steps)
 {
@@ -559,7 +558,7 @@ static int resident_steps(const Problem &p, int grid)
     if (2 * most > nw)
         return 0;
     const int steps = div_up(p.max_conns, column_split(most, nw));
-    return resident_bytes<TK, D>(steps) <= kResidentSmem ? steps : 0;
+    return resident_bytes<TK, D>(steps) <= kDynamicSmem ? steps : 0;
 }
 
 // Waits for the CG launch between the handle's two events and reads its status words.
@@ -647,8 +646,7 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     {
         s.steps = resident_steps<TK, D>(p, grid);
         const size_t smem = resident_bytes<TK, D>(s.steps);
-        if ((e = cudaFuncSetAttribute(k_cg<TK, TV, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        if ((e = allow_dynamic_smem((const void *)k_cg<TK, TV, D, true>)) != cudaSuccess)
             return e;
         e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D, true>, dim3(grid), dim3(kCGThreads), args, smem,
                                         p.stream);

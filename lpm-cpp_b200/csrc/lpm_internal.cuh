@@ -20,6 +20,15 @@ constexpr int kMaxCand = 512;    // connection candidates per particle before so
 constexpr double kEps = 1e-6;    // include/lpm.h:41
 constexpr int kSlice = 32;       // rows per slice of the sliced-ELL stiffness layout
 
+// Dynamic shared memory that the kernels whose need depends on the problem are allowed; what a launch takes
+// is its own.  The allowance belongs to the function on its device and is shared by all host threads, so
+// every launch sets the same one: a smaller problem's would refuse a larger one's launch on another thread.
+constexpr size_t kDynamicSmem = 176 * 1024;
+inline cudaError_t allow_dynamic_smem(const void *kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynamicSmem);
+}
+
 // std::max semantics ((a < b) ? b : a), which keeps the first argument when b is NaN
 __host__ __device__ inline double std_max(double a, double b) { return (a < b) ? b : a; }
 

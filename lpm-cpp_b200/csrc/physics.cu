@@ -359,8 +359,7 @@ cudaError_t launch_geometry_force(Problem &p)
     const size_t smem = geo_smem(p);
     if (smem > 48 * 1024)
     {
-        const cudaError_t e = cudaFuncSetAttribute(k_geometry_force, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem);
+        const cudaError_t e = allow_dynamic_smem((const void *)k_geometry_force);
         if (e != cudaSuccess)
             return e;
     }
@@ -396,8 +395,7 @@ cudaError_t launch_update_rr_impl(Problem &p, bool accumulate_reaction)
     const size_t smem = force_smem(p);
     if (smem > 48 * 1024)
     {
-        const cudaError_t e = cudaFuncSetAttribute(k_internal_force, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem);
+        const cudaError_t e = allow_dynamic_smem((const void *)k_internal_force);
         if (e != cudaSuccess)
             return e;
     }
