@@ -121,6 +121,7 @@ struct Problem
     double *partials = nullptr;       // kMaxGridBlocks * 4
     Scalars *scal = nullptr;
     Scalars *scal_host = nullptr;     // pinned mirror
+    uint64_t pinned_ctx = 0;          // the context of the pinned records (memory.cu)
     unsigned *barrier = nullptr;      // [0] count, [1] generation
     int64_t *cg_info = nullptr;       // device CG status words
     int64_t *cg_info_host = nullptr;  // pinned mirror
@@ -272,8 +273,8 @@ cudaError_t pool_alloc(T **ptr, size_t bytes, cudaStream_t st)
     *ptr = static_cast<T *>(v);
     return e;
 }
-cudaError_t pinned_take(void **ptr);
-void pinned_give(void *ptr);
+cudaError_t pinned_take(void **ptr, uint64_t *ctx);
+void pinned_give(void *ptr, uint64_t ctx);
 
 template <typename T>
 cudaError_t dalloc(Problem &p, T **ptr, size_t count)

@@ -669,7 +669,7 @@ static void free_problem(Problem &p)
     if (p.stream)
         cudaStreamSynchronize(p.stream);
     if (p.scal_host)
-        pinned_give(p.scal_host);
+        pinned_give(p.scal_host, p.pinned_ctx);
     for (auto &e : p.ev)
         if (e)
             cudaEventDestroy(e);
@@ -755,7 +755,7 @@ int32_t lpmgpu_create(const lpmgpu_desc *d, lpmgpu_solver **out)
         kntv(p.cell, d->plane_stress, d->E, d->mu, p.kntv);
     const size_t n = p.n;
     void *pinned = nullptr;
-    CKF(pinned_take(&pinned));
+    CKF(pinned_take(&pinned, &p.pinned_ctx));
     p.scal_host = static_cast<Scalars *>(pinned);
     p.cg_info_host = reinterpret_cast<int64_t *>(static_cast<char *>(pinned) + 128);
     std::memset(pinned, 0, 256);
