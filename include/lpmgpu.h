@@ -259,8 +259,9 @@ int32_t lpmgpu_fatigue_cycle(lpmgpu_solver *h, const lpmgpu_load_step *steps, in
 /* Autotuner of the CG launch shape (no counterpart in the reference; the reference's MKL CG has no
  * launch shape).  lpmgpu_autotune re-assembles K from the current state (call it between load
  * steps, after the first, so that the displacement BCs make K definite), then times `iterations` CG iterations of this problem's matrix (the FP32 inner solve in
- * mixed precision) for each candidate grid size: the default (one block per SM; for a problem that
- * solves in one cluster, its CTAs) and 3/4, 1/2, 1/4, 1/8, 1/16 of it.  The fastest stays in force for this handle's later
+ * mixed precision) for each candidate grid size: the default (one block per SM, at most one per
+ * slice; for a problem whose bond form runs in one cluster, its CTAs), timed in the form that it runs
+ * in, and 3/4, 1/2, 1/4, 1/8, 1/16 of it.  The fastest stays in force for this handle's later
  * solves; results then differ from the default grid's only by the rounding of the reductions.
  * lpmgpu_set_cg_grid sets the grid directly (0 = the default; values above the default are
  * clamped to it). */

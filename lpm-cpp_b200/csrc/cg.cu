@@ -689,6 +689,22 @@ static cudaError_t run_bond(Problem &p, const TV *b, TV *x, TV *r, TV *pa, TV *p
     return finish_cg(p, what, out, rr_final, declined);
 }
 
+// K x = b on the assembled matrix: small 2D FP64 problems in one cluster, the others on the grid
+template <typename TK, typename TV, int D>
+static cudaError_t run_assembled(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV *pa, TV *pb, TV *q, double rtol,
+                                 double atol, double abs_stop, int64_t maxit, CGResult &out, double *rr_final)
+{
+    if constexpr (D == 2 && sizeof(TV) == 8)
+        if (sell_cluster_fits(p))
+        {
+            cudaError_t e = cudaEventRecord(p.cg_ev[0], p.stream);
+            if (e == cudaSuccess)
+                e = enqueue_sell_cluster(p, b, x, rtol, atol, abs_stop, maxit);
+            return e != cudaSuccess ? e : finish_cg(p, "assembled fp64 cluster", out, rr_final, nullptr);
+        }
+    return run_cg<TK, TV, D>(p, K, b, x, r, pa, pb, q, rtol, atol, abs_stop, maxit, out, rr_final);
+}
+
 template <int D>
 static cudaError_t solve_dim(Problem &p, CGResult &out)
 {
@@ -707,17 +723,9 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
             return e;
         }
     }
-    if constexpr (D == 2)
-        if (p.desc.precision != LPMGPU_MIXED && sell_cluster_fits(p))
-        {
-            cudaError_t e = cudaEventRecord(p.cg_ev[0], p.stream);
-            if (e == cudaSuccess)
-                e = enqueue_sell_cluster(p, p.res, p.x, p.desc.cg_rtol, p.desc.cg_atol, -1.0, maxit);
-            return e != cudaSuccess ? e : finish_cg(p, "assembled fp64 cluster", out, nullptr, nullptr);
-        }
     if (p.desc.precision != LPMGPU_MIXED)
-        return run_cg<double, double, D>(p, p.K, p.res, p.x, p.r, p.p0, p.p1, p.q, p.desc.cg_rtol, p.desc.cg_atol,
-                                         -1.0, maxit, out, nullptr);
+        return run_assembled<double, double, D>(p, p.K, p.res, p.x, p.r, p.p0, p.p1, p.q, p.desc.cg_rtol,
+                                                p.desc.cg_atol, -1.0, maxit, out, nullptr);
     // FP32 Krylov solve inside FP64 iterative refinement on the same stopping rule
     cudaError_t e;
     // rr0 = ||b||^2 via r = b - K*0
@@ -871,7 +879,7 @@ static cudaError_t tune_dim(Problem &p, int iterations, lpmgpu_tune_result *res,
                 e2 = run_bond<TV>(p, b, x, r, pa, pb, 0.0, 0.0, 0.0, iterations, cr, nullptr, &off);
         }
         if (e2 == cudaSuccess && off)
-            e2 = run_cg<TK, TV, D>(p, K, b, x, r, pa, pb, q, 0.0, 0.0, 0.0, iterations, cr, nullptr);
+            e2 = run_assembled<TK, TV, D>(p, K, b, x, r, pa, pb, q, 0.0, 0.0, 0.0, iterations, cr, nullptr);
         return e2;
     };
     cudaError_t e = cudaSuccess;
@@ -901,7 +909,7 @@ static cudaError_t tune_dim(Problem &p, int iterations, lpmgpu_tune_result *res,
     res->ncandidates = (int32_t)cand.size();
     for (size_t k = 0; k < cand.size(); ++k)
     {
-        p.cg_grid = cand[k];
+        p.cg_grid = cand[k] == g0 ? 0 : cand[k]; // the default's own form is the one timed for it
         double us = 0;
         for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep)
         {
