@@ -1444,6 +1444,7 @@ cudaError_t enqueue_bond_cluster(Problem &p, const double *b, double *x, double 
     s.r = s.pa = s.pb = nullptr;
     const int nc = cluster_ctas(p);
     int G = div_up(p.bo_ng, nc), slots = G * p.bo_width, held = held_rows(p, nc);
+    p.cg_form = "cluster";
     void *args[] = {&s, &G, &slots, &held};
     if ((e = launch_cluster(cluster_kernel(p), nc, 32 * (G + 1), cluster_smem_of(p, G, held), args, p.stream)) != cudaSuccess)
         return e;
@@ -1474,10 +1475,12 @@ static cudaError_t launch_grid(Problem &p, BondCG<TV> &s)
         grid = p.cg_grid;
     void *args[] = {&s};
     bool staged = false;
+    p.cg_form = "general";
     if constexpr (!GEN)
         if (staged_fits(p, grid, sizeof(TV)))
         {
             staged = true;
+            p.cg_form = "staged";
             if ((e = cudaFuncSetAttribute(k_cg_bond<TV, D, GEN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kStagedSmem)) != cudaSuccess)
                 return e;

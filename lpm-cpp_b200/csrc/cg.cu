@@ -585,8 +585,8 @@ static cudaError_t finish_cg(Problem &p, const char *what, CGResult &out, double
             p.ctr.cg_kernel_seconds += ms * 1e-3;
         static const bool log = std::getenv("LPMGPU_LOG") != nullptr;
         if (log)
-            std::fprintf(stderr, "lpmgpu cg launch %lld: %s/%dd n=%d iters=%lld ms=%.3f\n", (long long)p.ctr.cg_launches,
-                         what, p.dim, p.n, (long long)p.cg_info_host[0], ms);
+            std::fprintf(stderr, "lpmgpu cg launch %lld: %s %s/%dd n=%d iters=%lld ms=%.3f\n",
+                         (long long)p.ctr.cg_launches, what, p.cg_form, p.dim, p.n, (long long)p.cg_info_host[0], ms);
     }
     if (p.cg_info_host[1] & 1)
         out.maxit_hits++;
@@ -636,6 +636,7 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     // the streamed form where every block has more than half a slice per warp, so no columns are split
     if (sizeof(TV) == 4 && D == 3 && 2 * (p.nslices / grid) > kCGThreads / 32)
     {
+        p.cg_form = "streamed";
         if ((e = cudaFuncSetAttribute(k_cg_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem)) !=
             cudaSuccess)
             return e;
@@ -644,6 +645,7 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
     }
     else if (resident_steps<TK, D>(p, grid) > 0)
     {
+        p.cg_form = "resident";
         s.steps = resident_steps<TK, D>(p, grid);
         const size_t smem = resident_bytes<TK, D>(s.steps);
         if ((e = allow_dynamic_smem((const void *)k_cg<TK, TV, D, true>)) != cudaSuccess)
@@ -652,8 +654,11 @@ static cudaError_t run_cg(Problem &p, const TK *K, const TV *b, TV *x, TV *r, TV
                                         p.stream);
     }
     else
+    {
+        p.cg_form = "general";
         e = cudaLaunchCooperativeKernel((const void *)k_cg<TK, TV, D, false>, dim3(grid), dim3(kCGThreads), args, 0,
                                         p.stream);
+    }
     if (e != cudaSuccess)
         return e;
     p.ctr.kernel_launches++;
@@ -675,10 +680,7 @@ static cudaError_t run_bond(Problem &p, const TV *b, TV *x, TV *r, TV *pa, TV *p
     if constexpr (sizeof(TV) == 8)
     {
         if (bond_cluster_fits(p))
-        {
-            what = "bond fp64 cluster";
             e = enqueue_bond_cluster(p, b, x, rtol, atol, abs_stop, maxit);
-        }
         else
             e = enqueue_bond_grid<TV>(p, b, x, r, pa, pb, rtol, atol, abs_stop, maxit);
     }
@@ -700,7 +702,7 @@ static cudaError_t run_assembled(Problem &p, const TK *K, const TV *b, TV *x, TV
             cudaError_t e = cudaEventRecord(p.cg_ev[0], p.stream);
             if (e == cudaSuccess)
                 e = enqueue_sell_cluster(p, b, x, rtol, atol, abs_stop, maxit);
-            return e != cudaSuccess ? e : finish_cg(p, "assembled fp64 cluster", out, rr_final, nullptr);
+            return e != cudaSuccess ? e : finish_cg(p, "assembled fp64", out, rr_final, nullptr);
         }
     return run_cg<TK, TV, D>(p, K, b, x, r, pa, pb, q, rtol, atol, abs_stop, maxit, out, rr_final);
 }

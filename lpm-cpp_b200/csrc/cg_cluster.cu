@@ -440,6 +440,7 @@ cudaError_t enqueue_sell_cluster(Problem &p, const double *b, double *x, double 
     s.maxit = maxit;
     s.info = p.cg_info;
     s.wait_ns = p.wait_ns;
+    p.cg_form = "cluster";
     void *args[] = {&s};
     e = launch_cluster((const void *)k_cg_sell_cluster, nc, kThreads, sell_smem(s.nslices, s.per, s.width), args, p.stream);
     if (e == cudaSuccess)

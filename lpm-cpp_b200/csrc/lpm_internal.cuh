@@ -125,6 +125,7 @@ struct Problem
     unsigned *barrier = nullptr;      // [0] count, [1] generation
     int64_t *cg_info = nullptr;       // device CG status words
     int64_t *cg_info_host = nullptr;  // pinned mirror
+    const char *cg_form = "";         // of the last CG launch, for the log
     // timing
     cudaEvent_t ev[8];
     double phase_s[4] = {0, 0, 0, 0};
