@@ -393,7 +393,8 @@ typedef struct
                                     slices of 32 rows per block: 1, 2 single reduction with 1 or 2 SpMV steps
                                     in flight, 3 single reduction with the matrix streamed into
                                     shared memory by bulk copies, 0 two reductions (the batch's tuner
-                                    picks it over its first launches unless LPMGPU_BATCH_SR fixes it) */
+                                    picks it over its first launches unless LPMGPU_BATCH_SR fixes it; with
+                                    that set, mixed members that fit one cluster use it too) */
     int32_t fp32_kernel_small;   /* the same for smaller launches */
     int32_t fp32_tuning;         /* 1 while the tuner is still trying the kernels */
     int32_t pad;

@@ -38,6 +38,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "bulk_copy.cuh"
@@ -2907,6 +2908,8 @@ struct lpmgpu_batch
             for (auto &L : lanes)
                 if (L->inflight && lane_ready(*L))
                     progressed = true; // the next round takes its results
+            if (!progressed)
+                std::this_thread::yield(); // as a wait of the runtime does where cores are short
         }
         if (!progressed && launched == 0)
         {
