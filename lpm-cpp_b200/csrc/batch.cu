@@ -2523,7 +2523,7 @@ struct lpmgpu_batch
     int32_t finish_linear(Member &m)
     {
         Problem &p = P(m);
-        cudaError_t e = launch_add_disp(p);
+        cudaError_t e = launch_add_disp(p, m.solving);
         if (e == cudaSuccess)
             e = enqueue_force_state(p, true);
         if (e != cudaSuccess)

@@ -222,7 +222,8 @@ cudaError_t launch_edamage_update(Problem &p);
 cudaError_t launch_hcf_init(Problem &p);
 cudaError_t launch_hcf_update(Problem &p);
 cudaError_t launch_fatigue_damage(Problem &p, double dNdt);
-cudaError_t launch_add_disp(Problem &p);        // xyz += x (solveLinearSystem position update)
+// xyz += x (solveLinearSystem position update); unseen: behind a solve whose status is not known yet
+cudaError_t launch_add_disp(Problem &p, bool unseen = false);
 cudaError_t launch_export_ref(const Problem &p, int64_t *IK, int64_t *JK, double *K); // device outputs
 cudaError_t launch_apply_bc(Problem &p, const lpmgpu_load_step &s);
 

@@ -78,3 +78,38 @@ def test_direct_solve():
         got, _ = g.solve_direct()
         assert np.array_equal(got, want)
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ns", [1, 300, 600, 1000, 1500, 2000, 3000])
+def test_batch_member(ns):
+    """A batch member whose cluster solve times out, at once or on the way, is left between two Newton
+    iterations: without the unfinished increment that the update behind the solve would add.  The states
+    there may be are those of the same iterations driven one by one."""
+    case = _block(L.Hexagon2D, 6.0)
+    ref = LPM.GpuProblem(case.assembly(), **TIGHT)
+    ref.apply_load_step(case.load_step(0))
+    ref.assemble(True)
+    states = [ref.state(("xyz",))["xyz"]]
+    for _ in range(8):
+        ref.update_force_state()
+        ref.update_rr()
+        u = np.zeros_like(case.xyz)
+        u[:, :case.dim] = ref.solve_linear()[0].reshape(case.n, case.dim)
+        states.append(states[-1] + u)
+        ref.set_xyz(states[-1])
+    ref.close()
+    for _ in range(5):
+        g = LPM.GpuProblem(case.assembly(), **TIGHT)
+        g.set_wait_limit_ns(ns)
+        batch = LPM.Batch()
+        mid = batch.add(g, [case.load_step(0)])
+        batch.run()
+        info = batch.member(mid)
+        assert info["state"] in (1, 2) and (ns > 1 or info["state"] == 2)
+        if info["state"] == 2:
+            assert info["status"] == LPM.ERR_TIMEOUT
+            xyz = g.state(("xyz",))["xyz"]
+            assert any(np.array_equal(xyz, s) for s in states)
+        batch.close()
+        g.close()
