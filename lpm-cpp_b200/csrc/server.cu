@@ -105,11 +105,19 @@ int64_t estimate_bytes(const lpmgpu_desc &d)
     // the fast assembly's lists: at most nb^2 two-hop paths of 5 bytes, a count per slot, T and
     // Ts per bond, U and the row offset per particle
     per_particle += (int64_t)nb * nb * 5 + nc + (int64_t)nb * 16 + 56;
-    // the bond form of K: per bond (rows padded to the lanes that share them) a column, its source
-    // bond, the cosines and two coefficients; per particle theta, S, U, the self block and a mask
-    per_particle += (int64_t)(nb + 8) * (24 + 8 * dim) + 192;
-    if (d.precision == LPMGPU_MIXED)
-        per_particle += (int64_t)(nb + 8) * (8 + 4 * dim) + 96;
+    // the bond form of K, where setup_bond_op builds one (in 3D mixed precision only for a problem that one
+    // cluster of 16 CTAs may hold, 31 groups of 32 rows each): per bond (rows padded to the lanes that share
+    // them) a column, its source bond and the cosines; per particle theta, a mask and a share of the
+    // groups' reach; with per-bond coefficients two more values a bond, and S, U and the self block
+    if ((d.ptype == LPMGPU_ELASTIC || d.ptype == LPMGPU_J2) &&
+        (dim == 2 || d.precision != LPMGPU_MIXED || d.n <= 16 * 31 * 32))
+    {
+        const bool general = d.bond_kn || d.bond_tv || d.bond_damage;
+        const int64_t entries = nb + 8, rows = 4 * dim + dim * (dim + 1) / 2;
+        per_particle += entries * (8 + 8 * dim + (general ? 16 : 0)) + 36 + (general ? 8 * rows : 0);
+        if (d.precision == LPMGPU_MIXED && dim == 2)
+            per_particle += entries * (4 * dim + (general ? 8 : 0)) + 16 + (general ? 4 * rows : 0);
+    }
     if (d.nonlocal_cutoff_ratio > 0 && d.radius > 0)
     {
         // nonlocal lists: the particles within cutoff_ratio x nonlocal_L, counted for the densest
