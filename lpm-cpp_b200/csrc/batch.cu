@@ -2164,6 +2164,7 @@ struct Member
     // (Scalars::bond_flag) goes through the member's lane instead.
     bool cluster = false;
     bool solving = false; // such a solve is in flight
+    double reaction_sq = 0; // of the force state before it
     int64_t lane_cost() const { return solo || cluster ? 0 : cost; }
 };
 
@@ -2466,10 +2467,13 @@ struct lpmgpu_batch
             return fail_member(m, cuda_status(e, "batched cluster solve"));
         stats.cg_launches++;
         m.solving = true;
+        m.reaction_sq = p.scal_host->reaction_sq;
         return finish_linear(m);
     }
 
-    // its result, once the member's stream has run dry; false when the solve timed out
+    // Its result, once the member's stream has run dry.  False when the Newton update behind it was not
+    // made: the solve timed out, or a mixed member's reached the cap, which holds for each inner solve of a
+    // refinement (solve_dim's rule); the member then refines in its lane, as if this solve had not been.
     bool take_cluster_solve(Member &m)
     {
         Problem &p = P(m);
@@ -2481,18 +2485,34 @@ struct lpmgpu_batch
             cluster_seconds += ms * 1e-3;
         }
         const int64_t it = p.cg_info_host[0];
-        m.cur.cg_iters += it;
-        m.cur.cg_maxit_hits += (p.cg_info_host[1] & 1) ? 1 : 0;
-        m.cur.refinements += p.desc.precision == LPMGPU_MIXED ? 1 : 0; // one outer step, solved in FP64
-        m.dof_iters += it * (int64_t)p.n * p.dim;
+        const bool mixed = p.desc.precision == LPMGPU_MIXED;
         p.ctr.cg_iters += it;
         round_max_it = std::max(round_max_it, it);
         if (p.cg_info_host[1] & 2)
         {
+            m.cur.cg_iters += it;
+            m.dof_iters += it * (int64_t)p.n * p.dim;
             set_last_error("a device-side wait timed out in the batched cluster solve");
             fail_member(m, LPMGPU_ERR_TIMEOUT);
             return false;
         }
+        if (mixed && (p.cg_info_host[1] & 1) && !p.scal_host->err &&
+            std::isfinite(reinterpret_cast<const double *>(p.cg_info_host)[3]))
+        {
+            // the force state behind the solve saw the same positions; its reactions count once
+            p.scal_host->reaction_sq = m.reaction_sq;
+            const cudaError_t e = cudaMemcpyAsync(&p.scal->reaction_sq, &p.scal_host->reaction_sq, sizeof(double),
+                                                  cudaMemcpyHostToDevice, p.stream);
+            if (e != cudaSuccess)
+                fail_member(m, cuda_status(e, "batched refinement"));
+            else
+                start_refinement(m);
+            return false;
+        }
+        m.cur.cg_iters += it;
+        m.dof_iters += it * (int64_t)p.n * p.dim;
+        m.cur.cg_maxit_hits += (p.cg_info_host[1] & 1) ? 1 : 0;
+        m.cur.refinements += mixed ? 1 : 0; // one outer step, solved in FP64
         return true;
     }
 
@@ -2506,6 +2526,13 @@ struct lpmgpu_batch
             m.ph = Ph::NeedCG; // a solo member's solve sets up its own refinement
             return LPMGPU_OK;
         }
+        return start_refinement(m);
+    }
+
+    // a mixed member's refinement in its lane; the residual's square is in its scalar record
+    int32_t start_refinement(Member &m)
+    {
+        Problem &p = P(m);
         m.ir_rr = p.scal_host->res_sq;
         m.ir_stop = p.desc.cg_rtol * m.ir_rr + p.desc.cg_atol;
         cudaError_t e = cudaMemsetAsync(p.x, 0, sizeof(double) * (size_t)p.n * p.dim, p.stream);
@@ -2523,7 +2550,8 @@ struct lpmgpu_batch
     int32_t finish_linear(Member &m)
     {
         Problem &p = P(m);
-        cudaError_t e = launch_add_disp(p, m.solving);
+        // behind a cluster solve: not after a timeout, and not after a mixed member's cap
+        cudaError_t e = launch_add_disp(p, !m.solving ? 0 : p.desc.precision == LPMGPU_MIXED ? 3 : 2);
         if (e == cudaSuccess)
             e = enqueue_force_state(p, true);
         if (e != cudaSuccess)

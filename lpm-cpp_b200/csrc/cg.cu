@@ -716,13 +716,21 @@ static cudaError_t solve_dim(Problem &p, CGResult &out)
     if (p.bo_valid && (p.desc.precision != LPMGPU_MIXED || bond_cluster_fits(p)))
     {
         // Mixed precision in the cluster form: its bonds are in shared memory and its iterations are
-        // bound by latency, not by bytes, so the correction is solved for in FP64 at once.
+        // bound by latency, not by bytes, so the correction is solved for in FP64 at once.  The caller's
+        // cap, though, holds for each inner solve of a refinement, which goes on from one that reached it:
+        // then the refinement below is run instead, as if this solve had not been.
+        CGResult at_once;
+        double rr = 0.0;
         const cudaError_t e = run_bond<double>(p, p.res, p.x, p.r, p.p0, p.p1, p.desc.cg_rtol, p.desc.cg_atol, -1.0,
-                                               maxit, out, nullptr, &declined);
-        if (e != cudaSuccess || !declined)
-        {
-            out.refinements += p.desc.precision == LPMGPU_MIXED ? 1 : 0;
+                                               maxit, at_once, &rr, &declined);
+        if (e != cudaSuccess)
             return e;
+        const bool mixed = p.desc.precision == LPMGPU_MIXED;
+        if (!declined && !(mixed && at_once.maxit_hits > 0 && std::isfinite(rr)))
+        {
+            out = at_once;
+            out.refinements += mixed ? 1 : 0;
+            return cudaSuccess;
         }
     }
     if (p.desc.precision != LPMGPU_MIXED)

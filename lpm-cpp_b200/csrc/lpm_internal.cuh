@@ -222,8 +222,9 @@ cudaError_t launch_edamage_update(Problem &p);
 cudaError_t launch_hcf_init(Problem &p);
 cudaError_t launch_hcf_update(Problem &p);
 cudaError_t launch_fatigue_damage(Problem &p, double dNdt);
-// xyz += x (solveLinearSystem position update); unseen: behind a solve whose status is not known yet
-cudaError_t launch_add_disp(Problem &p, bool unseen = false);
+// xyz += x (solveLinearSystem position update); skip: the status bits of the solve before it, which the
+// host has not seen, that forbid it
+cudaError_t launch_add_disp(Problem &p, int skip = 0);
 cudaError_t launch_export_ref(const Problem &p, int64_t *IK, int64_t *JK, double *K); // device outputs
 cudaError_t launch_apply_bc(Problem &p, const lpmgpu_load_step &s);
 

@@ -530,20 +530,20 @@ cudaError_t launch_static_damage(Problem &p)
 }
 
 // Solver::solveLinearSystem position update (solver.h:101-108).  info: the status words of a solve whose
-// outcome the host has not seen; after one that timed out (bit 2) the positions stay as they are.
-__global__ void k_add_disp(int n, int dim, const double *__restrict__ x, const int64_t *__restrict__ info,
+// outcome the host has not seen; after one with a bit of `skip` the positions stay as they are.
+__global__ void k_add_disp(int n, int dim, const double *__restrict__ x, const int64_t *__restrict__ info, int skip,
                            double *__restrict__ xyz)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (info && (info[1] & 2)))
+    if (i >= n || (info && (info[1] & skip)))
         return;
     for (int k = 0; k < dim; ++k)
         xyz[3 * i + k] = xyz[3 * i + k] + (0.0 + x[(int64_t)dim * i + k]);
 }
 
-cudaError_t launch_add_disp(Problem &p, bool unseen)
+cudaError_t launch_add_disp(Problem &p, int skip)
 {
-    k_add_disp<<<div_up(p.n, 256), 256, 0, p.stream>>>(p.n, p.dim, p.x, unseen ? p.cg_info : nullptr, p.xyz);
+    k_add_disp<<<div_up(p.n, 256), 256, 0, p.stream>>>(p.n, p.dim, p.x, skip ? p.cg_info : nullptr, skip, p.xyz);
     p.ctr.kernel_launches++;
     return cudaGetLastError();
 }
