@@ -69,7 +69,7 @@ typedef struct
     int32_t max_iter;        /* Newton iteration cap (max_NR_iter) */
     double tol_iter;         /* Newton tolerance (tol_NR_iter) */
     double cg_rtol, cg_atol; /* squared-norm CG test ||r||^2 <= rtol*||r0||^2 + atol (solver.h:312-313) */
-    int64_t cg_maxit;        /* CG cap, 0 = problem size (solver.h:308) */
+    int64_t cg_maxit;        /* CG cap (mixed: of each inner solve), 0 = problem size (solver.h:308) */
     int32_t precision;       /* LPMGPU_FP64 or LPMGPU_MIXED */
     int32_t device;          /* CUDA device ordinal */
     /* Optional inputs (NULL = derive them as the reference's Assembly constructor would).

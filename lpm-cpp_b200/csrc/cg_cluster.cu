@@ -81,7 +81,7 @@ constexpr int kMaxCtas = 16;
 //
 // Bound by shared-memory bandwidth (the product reads 36 bytes per block, its 16 partial rows go
 // through memory, p and r are whole vectors) and by 60 cycles per level of each warp sum.  A plate of
-// 1,840 particles: 7.3 us per iteration on the grid, 5.7 here.
+// 1,840 particles: 6.9 us per iteration on the grid, 5.7 here; 1,050: 6.3 and 4.6.
 struct SellCG
 {
     int n, nslices, per, width; // most slices of a CTA, most block columns of a slice

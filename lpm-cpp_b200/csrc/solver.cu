@@ -206,9 +206,9 @@ static int32_t linear_solve_direct(Problem &p, lpmgpu_stats *st, bool *used)
 // One linear solve K x = res.  desc.direct 1: the band Cholesky.  desc.direct 2 (the drop-ins'
 // SolverMode::PARDISO): the CG at the caller's tolerance first, and the band Cholesky only when
 // the CG reached its cap or broke down.  Measured on B200 (hexagonal plates of 2,900 and 11,500
-// particles, one factorisation and three solves per load step): the band solve took 20x and 58x
-// the CG's time per load step, so the CG serves PARDISO mode and the factorisation is kept for
-// the systems the CG cannot solve.
+// particles, one factorisation and three solves per load step): the band solve takes 2.0x and 3.8x
+// the CG's time per load step (6.5 against 3.2 ms, 38 against 9.9 ms), so the CG serves PARDISO mode
+// and the factorisation is kept for the systems the CG cannot solve.
 static int32_t linear_solve(Problem &p, lpmgpu_stats *st)
 {
     bool direct = false;
