@@ -530,13 +530,20 @@ cudaError_t launch_static_damage(Problem &p)
 }
 
 // Solver::solveLinearSystem position update (solver.h:101-108).  info: the status words of a solve whose
-// outcome the host has not seen; after one with a bit of `skip` the positions stay as they are.
+// outcome the host has not seen; after one with a bit of `skip` the positions stay as they are (after a
+// capped one, bit 1, only if it left a finite residual, which a refinement can start from).
 __global__ void k_add_disp(int n, int dim, const double *__restrict__ x, const int64_t *__restrict__ info, int skip,
                            double *__restrict__ xyz)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (info && (info[1] & skip)))
+    if (i >= n)
         return;
+    if (info)
+    {
+        const int64_t st = info[1] & skip;
+        if ((st & 2) || ((st & 1) && isfinite(reinterpret_cast<const double *>(info)[3])))
+            return;
+    }
     for (int k = 0; k < dim; ++k)
         xyz[3 * i + k] = xyz[3 * i + k] + (0.0 + x[(int64_t)dim * i + k]);
 }
