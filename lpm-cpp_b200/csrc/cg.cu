@@ -575,6 +575,7 @@ static cudaError_t finish_cg(Problem &p, const char *what, CGResult &out, double
     if (declined && (p.cg_info_host[1] & kBondDeclined))
     {
         *declined = true;
+        p.bo_valid = false; // so does every other solve with this K
         return cudaSuccess;
     }
     out.iters += p.cg_info_host[0];
